@@ -170,6 +170,8 @@ StepArgs base_args(const ouc_ctx* c) {
     a.box_map = c->box_map;
     a.own_map = c->own_map;
     a.s_map = c->s_map;
+    a.mid_map = c->mid_map;
+    for (int k = 0; k < 2; ++k) a.small_map[k] = c->small_map[k];
     a.state0 = c->box_state0;
     a.fstride = c->fstride;
     a.nfields = kFieldsPerShot;
@@ -422,9 +424,18 @@ int rcv_step(ouc_ctx* ctx, StepArgs& ar, Side& r, int n, int t, cudaStream_t st 
 // from levels t+1 and t+2 with the strip restore, and the imaging condition
 // (PS:2326-2361).  At t = nt-1 there is no reconstruction: the forward's
 // final level is correlated as it stands.
-int rec_step(ouc_ctx* ctx, StepArgs& as, Side& s, const Side& r, int n, int t, bool exact_strips, bool theta_src) {
+void bind_rec(const ouc_ctx* ctx, StepArgs& as, const Side& s, const Side& r, int t, bool exact_strips, bool theta_src) {
     const int nt = ctx->nt;
-    if (t == nt - 1) {
+    bind_side(as, s);
+    as.t = t;
+    as.src_recon = theta_src && (exact_strips || t + 1 == nt - 1);
+    as.slot_u = exact_strips ? t : (t + 1 == nt - 1 ? nt - 2 : t + 1);
+    as.slot_s = t + 1;
+    for (int k = 0; k < 4; ++k) as.rcv[k] = r.now[k];
+}
+
+int rec_step(ouc_ctx* ctx, StepArgs& as, Side& s, const Side& r, int n, int t, bool exact_strips, bool theta_src) {
+    if (t == ctx->nt - 1) {
         StepArgs ai = base_args(ctx);
         for (int k = 0; k < 4; ++k) { ai.now[k] = s.now[k]; ai.rcv[k] = r.now[k]; }
         for (int k = 0; k < 3; ++k) ai.acc[k] = ctx->acc[k];
@@ -433,12 +444,7 @@ int rec_step(ouc_ctx* ctx, StepArgs& as, Side& s, const Side& r, int n, int t, b
         s.swap_levels();   // now = level NT-1, past = level NT
         return OUC_OK;
     }
-    bind_side(as, s);
-    as.t = t;
-    as.src_recon = theta_src && (exact_strips || t + 1 == nt - 1);
-    as.slot_u = exact_strips ? t : (t + 1 == nt - 1 ? nt - 2 : t + 1);
-    as.slot_s = t + 1;
-    for (int k = 0; k < 4; ++k) as.rcv[k] = r.now[k];
+    bind_rec(ctx, as, s, r, t, exact_strips, theta_src);
     if (launch_step(ctx->N, kRec, as, ctx->rec_tiles_x, n, ctx->stream))
         return fail(ctx, OUC_EINVAL, "step launch refused (half-order or state map)");
     s.swap_levels();
@@ -481,6 +487,36 @@ int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src) {
     if (ctx->cfg.gradient) CK(cudaMemsetAsync(ctx->grad, 0, (size_t)n * 3 * ctx->fstride * sizeof(float), ctx->stream));
     StepArgs ar = rcv_args(ctx);
     StepArgs as = rec_args(ctx);
+    Tier tier = kAuto;
+    if (ctx->seg_rows == 0) tier = pick_tier(ctx->N, &as, &ar, kRcv, n);
+    ar.tier = as.tier = tier;
+    if (tier >= kSmall24) {
+        // Small launches: one per back-step holds the reconstruction +
+        // imaging of step t+1 and the receiver step t, which are independent
+        // (k_small_back).  The gradient of step t+1 reads both sides first.
+        if ((rc = rcv_step(ctx, ar, r, n, ctx->nt - 1))) return rc;
+        for (int t = ctx->nt - 2; t >= 0; --t) {
+            if (ctx->cfg.gradient) grad_step(ctx, s, r, n, t + 1);
+            if (t == ctx->nt - 2) {   // no reconstruction at the last level
+                if ((rc = rec_step(ctx, as, s, r, n, t + 1, exact_strips, theta_src))) return rc;
+                if ((rc = rcv_step(ctx, ar, r, n, t))) return rc;
+                continue;
+            }
+            bind_rec(ctx, as, s, r, t + 1, exact_strips, theta_src);
+            bind_side(ar, r);
+            ar.t = t;
+            if (launch_back(ctx->N, as, ar, n, ctx->stream))
+                return fail(ctx, OUC_EINVAL, "step launch refused (half-order or state map)");
+            s.swap_levels();
+            r.swap_levels();
+            r.swap_memory();
+            ctx->timing.kernel_launches += 1;
+        }
+        if (ctx->cfg.gradient) grad_step(ctx, s, r, n, 0);
+        if ((rc = rec_step(ctx, as, s, r, n, 0, exact_strips, theta_src))) return rc;
+        CK(cudaGetLastError());
+        return OUC_OK;
+    }
     if (ctx->cfg.gradient || !ctx->stream2) {
         for (int t = ctx->nt - 1; t >= 0; --t) {
             if ((rc = rcv_step(ctx, ar, r, n, t))) return rc;
@@ -868,6 +904,8 @@ int ouc_create(const ouc_config* cfg, const float* vp, const float* vs, const fl
         ctx->box_map = m.box_map;
         ctx->own_map = m.own_map;
         ctx->s_map = m.s_map;
+        ctx->mid_map = m.mid_map;
+        for (int k = 0; k < 2; ++k) ctx->small_map[k] = m.small_map[k];
         ctx->box_state0 = m.state0;
     }
     // kernel attributes set before any graph capture

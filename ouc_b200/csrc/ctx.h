@@ -49,6 +49,8 @@ struct ouc_ctx {
     alignas(64) CUtensorMap box_map;   // tensor map of the state block (StepArgs::box_map)
     alignas(64) CUtensorMap own_map;   // and its own-cell box form (StepArgs::own_map)
     alignas(64) CUtensorMap s_map;     // and its S-region box form (StepArgs::s_map)
+    alignas(64) CUtensorMap mid_map;   // and the U boxes of the 16 x 64 tiles (StepArgs::mid_map)
+    alignas(64) CUtensorMap small_map[2];   // and of the small tiles (StepArgs::small_map)
     const float* box_state0 = nullptr;  // its start (null until encoded)
     size_t shot_stride = 0;      // floats per shot block (kFieldsPerShot fields)
     int tiles_x = 0, tiles_z = 0;

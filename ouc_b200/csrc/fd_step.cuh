@@ -20,6 +20,10 @@
 // Receiver extraction, record injection, boundary-strip save/restore and the
 // zero-lag imaging condition ride along in the same launch.
 //
+// The same code runs on 16 x 64 tiles (MidGeo) where a launch has too few
+// 32 x 64 ones to fill its waves; launches smaller still use fd_small.cuh
+// (pick_tier in kernels.cu chooses, with the measurements).
+//
 // Cost structure.  Tiles whose whole neighbourhood lies inside the update
 // domain, away from the boundary ring, the source and the receiver row are
 // "clean" and run no per-cell test at all; the few "edge" tiles mask per
@@ -51,11 +55,18 @@
 
 namespace ouc {
 
-template <int N>
+// Geometry of a tile of TX x 64 cells worked on by 256 threads: TX = 32, or
+// 16 for launches that do not fill the GPU with the larger tiles (MidGeo).
+template <int N_, int TX_ = 32>
 struct TileGeo {
-    static constexpr int TX = 32;                  // tile rows (x)
+    static constexpr int N = N_;
+    static constexpr bool small = false, mid = TX_ < 32;
+    static constexpr int TX = TX_;                 // tile rows (x)
     static constexpr int TZ = 64;                  // tile columns (z)
-    static constexpr int SHX = (N + 1) & ~1;       // S-stage row halo (even)
+    static constexpr int NT = kThreads;
+    static constexpr int RS = TX / 8;              // rows of an S item
+    static constexpr int RU = TX / 16;             // rows of a U item
+    static constexpr int SHX = (N + RS / 2 - 1) / (RS / 2) * (RS / 2);   // S-stage row halo (SR a multiple of RS)
     static constexpr int HS = (N + 3) & ~3;        // S-stage column halo (float4 aligned)
     static constexpr int HU = (HS + N + 3) & ~3;   // U column halo
     static constexpr int NB = (N + 3) / 4;         // float4 blocks on each side of a z window
@@ -73,12 +84,14 @@ struct TileGeo {
     static constexpr int oQzx = oQxx + TX * SC;
     static constexpr int floats = oQzx + TX * SC;
     static constexpr int bytes = floats * 4;
-    static constexpr int itemsA = (SR / 4) * (TZ / 4);        // S items over all rows, own columns
-    static constexpr int itemsB = (TX / 4) * (2 * HS / 4);    // S items over own rows, halo columns
-    static_assert(SR % 4 == 0, "S rows must group by 4");
+    static constexpr int itemsA = (SR / RS) * (TZ / 4);       // S items over all rows, own columns
+    static constexpr int itemsB = (TX / RS) * (2 * HS / 4);   // S items over own rows, halo columns
+    static_assert(SR % RS == 0, "S rows group by RS");
     static_assert(itemsA + itemsB <= kThreads, "one S item per thread");
-    static_assert((TX / 2) * (TZ / 4) == kThreads, "one U item per thread");
+    static_assert((TX / RU) * (TZ / 4) == kThreads, "one U item per thread");
 };
+template <int N>
+using MidGeo = TileGeo<N, 16>;
 
 // ---- small helpers -----------------------------------------------------------
 __device__ __forceinline__ float4 ld4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -273,6 +286,10 @@ __device__ __forceinline__ void tma_box4(void* dst, const CUtensorMap* map, int 
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(b))
         : "memory");
 }
+// Fetch a tensor map (kernel argument) ahead of its first copy.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(reinterpret_cast<uint64_t>(map)) : "memory");
+}
 // L2 prefetch of one box of a 4-D tensor map (no shared-memory write, no
 // completion to wait for).  Same coordinate rule as tma_box4.
 __device__ __forceinline__ void tma_prefetch_box4(const CUtensorMap* map, int c0, int c1, int c2, int c3) {
@@ -281,6 +298,15 @@ __device__ __forceinline__ void tma_prefetch_box4(const CUtensorMap* map, int c0
                  "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
+// Programmatic dependent launch.  The step kernels are launched so that a
+// launch may start while the one before it in the stream still runs
+// (launch_pdl): they read launch constants (arguments, shot descriptors,
+// models, strips of earlier phases) first, let their own successor start at
+// once, and touch the wavefields only after pdl_wait, which returns when the
+// previous launch has completed and its writes are visible (at once when the
+// launch was an ordinary one).
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Per-launch, per-shot constants.
@@ -408,38 +434,58 @@ __device__ __forceinline__ bool rect_meets_ring(const Ring& R, int i0, int i1, i
     return meets_box && !inside_deep;
 }
 
+// The part of one ring band (a rectangle of the grid) inside a rectangle of
+// cells: ia, ja its corner, w its columns, n its cells; cell (i, j) has ring
+// index c + i * stride + j.
+struct BandPart {
+    int ia, ja, w, n, c, stride;
+};
+__device__ __forceinline__ BandPart band_part(const Ring& R, int b, int i0, int i1, int j0, int j1) {
+    const int L = R.L, N = R.N, X = R.X, Z = R.Z, n2 = 2 * N, W = R.W, hm = R.H - 4 * N;
+    const int bi0 = b == 3 ? X - L - N : L - N, bi1 = b == 2 ? L + N : X - L + N;
+    const int bj0 = b == 0 ? L - N : b == 1 ? Z - L - N : L + N;
+    const int bj1 = b == 0 ? L + N : b == 1 ? Z - L + N : Z - L - N;
+    const int base = b == 0 ? 0 : b == 1 ? W * n2 : b == 2 ? 2 * W * n2 : 2 * W * n2 + n2 * hm;
+    BandPart q;
+    q.stride = b < 2 ? n2 : hm;
+    q.ia = max(i0, bi0);
+    q.ja = max(j0, bj0);
+    const int h = min(i1, bi1) - q.ia;
+    q.w = min(j1, bj1) - q.ja;
+    q.n = h > 0 && q.w > 0 ? h * q.w : 0;
+    q.c = base - bi0 * q.stride - bj0;
+    return q;
+}
+
 // Visit, cooperatively over the CTA, the boundary-ring cells inside the
 // rectangle [i0, i1) x [j0, j1) (global coordinates): f(i, j, ring index).
-// The four bands are rectangles, so each visit is a plain 2-D loop and the
-// strip accesses are contiguous along z.
-template <class F>
+// The cells of all four bands form one index range, so that a tile that
+// meets several bands (a corner, a narrow grid) waits for its strip loads
+// once and not once per band; the strip accesses are contiguous along z.
+template <int NT = kThreads, class F>
 __device__ __forceinline__ void for_ring(const Ring& R, int i0, int i1, int j0, int j1, F&& f) {
-    const int L = R.L, N = R.N, X = R.X, Z = R.Z, n2 = 2 * N, W = R.W, hm = R.H - 4 * N;
-#pragma unroll 1
-    for (int b = 0; b < 4; ++b) {
-        int bi0, bi1, bj0, bj1, base, stride;
-        if (b == 0) { bi0 = L - N; bi1 = X - L + N; bj0 = L - N; bj1 = L + N; base = 0; stride = n2; }
-        else if (b == 1) { bi0 = L - N; bi1 = X - L + N; bj0 = Z - L - N; bj1 = Z - L + N; base = W * n2; stride = n2; }
-        else if (b == 2) { bi0 = L - N; bi1 = L + N; bj0 = L + N; bj1 = Z - L - N; base = 2 * W * n2; stride = hm; }
-        else { bi0 = X - L - N; bi1 = X - L + N; bj0 = L + N; bj1 = Z - L - N; base = 2 * W * n2 + n2 * hm; stride = hm; }
-        const int ia = max(i0, bi0), ib = min(i1, bi1), ja = max(j0, bj0), jb = min(j1, bj1);
-        if (ia >= ib || ja >= jb) continue;
-        const int w = jb - ja, n = (ib - ia) * w;
-        // k / w as a multiply-high by m = ceil(2^32 / w): exact for k < 2^16
-        // and w <= 2^16 (the error k (m - 2^32 / w) / 2^32 < 2^-16 stays
-        // below 1/w); the rectangles here hold well under 2^16 cells
-        const unsigned m = w > 1 ? 0xFFFFFFFFu / (unsigned)w + 1u : 0u;
-        for (int k = threadIdx.x; k < n; k += kThreads) {
-            const int q = w > 1 ? (int)__umulhi((unsigned)k, m) : k;
-            const int i = ia + q, j = ja + (k - q * w);
-            f(i, j, base + (i - bi0) * stride + (j - bj0));
-        }
+    const BandPart b0 = band_part(R, 0, i0, i1, j0, j1), b1 = band_part(R, 1, i0, i1, j0, j1);
+    const BandPart b2 = band_part(R, 2, i0, i1, j0, j1), b3 = band_part(R, 3, i0, i1, j0, j1);
+    const int e0 = b0.n, e1 = e0 + b1.n, e2 = e1 + b2.n, e3 = e2 + b3.n;
+    for (int k = threadIdx.x; k < e3; k += NT) {
+        const bool p0 = k < e0, p1 = k < e1, p2 = k < e2;
+        const int w = p0 ? b0.w : p1 ? b1.w : p2 ? b2.w : b3.w;
+        const int kk = k - (p0 ? 0 : p1 ? e0 : p2 ? e1 : e2);
+        // kk / w: the product is within (kk / w) 2^-22 of (kk + 1/2) / w, whose
+        // distance to a whole number is at least 1 / (2 w); exact for the
+        // few thousand cells of these rectangles
+        const int q = (int)(((float)kk + 0.5f) * (1.0f / (float)w));
+        const int i = (p0 ? b0.ia : p1 ? b1.ia : p2 ? b2.ia : b3.ia) + q;
+        const int j = (p0 ? b0.ja : p1 ? b1.ja : p2 ? b2.ja : b3.ja) + (kk - q * w);
+        const int c = p0 ? b0.c : p1 ? b1.c : p2 ? b2.c : b3.c;
+        const int stride = p1 ? b0.stride : b2.stride;
+        f(i, j, c + i * stride + j);
     }
 }
 
-template <int N, int MODE>
+template <class G, int MODE>
 __device__ __forceinline__ TileFlags tile_flags(const StepArgs& p, const Geo& gm, const ShotView& sv, int x0, int z0) {
-    using G = TileGeo<N>;
+    constexpr int N = G::N;
     const int X = gm.X, Z = p.Z, L = p.L;
     TileFlags f;
     f.px = f.pz = false;
@@ -476,9 +522,9 @@ __device__ __forceinline__ TileFlags tile_flags(const StepArgs& p, const Geo& gm
 // DRAM; prefetched at the tile's start, their latency runs under the U-box
 // copy and the S-stage instead of stalling the restore loops.  One 128-byte
 // line per prefetch, at element addresses inside the strip slots.
-template <int N>
+template <class G>
 __device__ __forceinline__ void prefetch_ring(const StepArgs& p, const Geo& gm, const ShotDesc& d, int x0, int z0) {
-    using G = TileGeo<N>;
+    constexpr int N = G::N;
     const Ring& R = gm.ring;
     const int L = R.L, X = R.X, Z = R.Z, n2 = 2 * R.N, W = R.W, hm = R.H - 4 * R.N;
     const int eb = strip_elem_bytes(p.strip_prec), per_line = 128 / eb;
@@ -502,7 +548,7 @@ __device__ __forceinline__ void prefetch_ring(const StepArgs& p, const Geo& gm, 
             const int per_f = rows * nl;
             const unsigned mf = per_f > 1 ? 0xFFFFFFFFu / (unsigned)per_f + 1u : 0u;
             const unsigned ml = nl > 1 ? 0xFFFFFFFFu / (unsigned)nl + 1u : 0u;
-            for (int k = threadIdx.x; k < nf * per_f; k += kThreads) {
+            for (int k = threadIdx.x; k < nf * per_f; k += G::NT) {
                 const int f = per_f > 1 ? (int)__umulhi((unsigned)k, mf) : k, rem = k - f * per_f;
                 const int row = nl > 1 ? (int)__umulhi((unsigned)rem, ml) : rem, l = rem - row * nl;
                 // element of the run: l * per_line < jb - ja
@@ -527,10 +573,9 @@ __device__ __forceinline__ bool u_live(const StepArgs& p, const Geo& gm, int gi,
 // model over the S region (phase 2), one 128-byte line per instruction
 // (every address inside the field allocations, guard rows and columns
 // included).  The U box of phase 1 arrives by tensor copies.
-template <int N, int MODE>
+template <class G, int MODE>
 __device__ __forceinline__ void prefetch_tile(const StepArgs& p, const Geo& gm, int x0, int z0, int slot,
                                               const TileFlags& fl) {
-    using G = TileGeo<N>;
     constexpr int TX = G::TX, TZ = G::TZ, SHX = G::SHX, HS = G::HS;
     const int tid = threadIdx.x;
     const int P = p.pitch;
@@ -575,6 +620,11 @@ __device__ __forceinline__ void prefetch_tile(const StepArgs& p, const Geo& gm, 
     }
 }
 
+template <class G>
+__device__ __forceinline__ const CUtensorMap* u_map(const StepArgs& p) {
+    return G::small ? &p.small_map[G::TX / 8 - 2] : G::mid ? &p.mid_map : &p.box_map;
+}
+
 // Issue the four tensor copies of a tile's U box (one thread): the UC x UR
 // box of each P/S field of the current level, completing on the CTA's
 // mbarrier -- P into the U arrays, S into the S-stage area, which is unused
@@ -583,9 +633,9 @@ __device__ __forceinline__ void prefetch_tile(const StepArgs& p, const Geo& gm, 
 // copies overlap the tile's set-up.  `slot` is the shot's index in the
 // launch, which is its slot in the state block (its fields lie slot x
 // shot_stride floats after shot 0's).
-template <int N>
+template <class G>
 __device__ __forceinline__ void issue_u_box(const StepArgs& p, float* sm, int x0, int z0, int slot, uint64_t* bar) {
-    using G = TileGeo<N>;
+    const CUtensorMap* map = u_map<G>(p);
     static_assert(G::floats - G::oTh >= 2 * G::UR * G::UC, "S staging fits the S-stage area");
     static_assert((G::oUz * 4) % 128 == 0 && (G::oTh * 4) % 128 == 0 && (G::UR * G::UC * 4) % 128 == 0,
                   "tensor-copy destinations are 128-byte aligned");
@@ -593,12 +643,12 @@ __device__ __forceinline__ void issue_u_box(const StepArgs& p, float* sm, int x0
     // a previous tile's shared-memory accesses (generic proxy) precede these writes
     fence_proxy_async();
     // allocation coordinates: column z0 - HU + kZOFF (a multiple of 4), row x0 - SHX - N + kGX (>= 0)
-    const int c0 = z0 - G::HU + kZOFF, c1 = x0 - G::SHX - N + kGX;
+    const int c0 = z0 - G::HU + kZOFF, c1 = x0 - G::SHX - G::N + kGX;
     float* stS = sm + G::oTh;
-    tma_box4(sm + G::oUx, &p.box_map, c0, c1, p.now_field[0], slot, bar);
-    tma_box4(sm + G::oUz, &p.box_map, c0, c1, p.now_field[1], slot, bar);
-    tma_box4(stS, &p.box_map, c0, c1, p.now_field[2], slot, bar);
-    tma_box4(stS + G::UR * G::UC, &p.box_map, c0, c1, p.now_field[3], slot, bar);
+    tma_box4(sm + G::oUx, map, c0, c1, p.now_field[0], slot, bar);
+    tma_box4(sm + G::oUz, map, c0, c1, p.now_field[1], slot, bar);
+    tma_box4(stS, map, c0, c1, p.now_field[2], slot, bar);
+    tma_box4(stS + G::UR * G::UC, map, c0, c1, p.now_field[3], slot, bar);
 }
 
 // Offsets within one field are 32-bit ints (row * pitch + column, guard rows
@@ -611,10 +661,10 @@ __device__ __forceinline__ void issue_u_box(const StepArgs& p, float* sm, int x0
 // bit 0 of *p.err set, when the copies did not land within the wait's bound
 // (or an earlier launch had recorded such a failure): the tile is then left
 // unwritten and the host reports OUC_ETIMEOUT after the call.
-template <int N, int MODE>
+template <class G, int MODE>
 __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, const ShotView& sv, float* sm, int x0, int z0,
                                           const TileFlags& f, uint64_t* bar, unsigned parity) {
-    using G = TileGeo<N>;
+    constexpr int N = G::N;
     constexpr int TX = G::TX, TZ = G::TZ, SHX = G::SHX, HS = G::HS, HU = G::HU, UC = G::UC, SC = G::SC;
     const int tid = threadIdx.x;
     const int P = p.pitch;
@@ -692,11 +742,11 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
         int r0, c;
         const bool groupA = tid < G::itemsA;
         if (groupA) {
-            r0 = -SHX + 4 * (tid / (TZ / 4));
+            r0 = -SHX + G::RS * (tid / (TZ / 4));
             c = 4 * (tid % (TZ / 4));
         } else {
             const int k = tid - G::itemsA;
-            r0 = 4 * (k / (2 * HS / 4));
+            r0 = G::RS * (k / (2 * HS / 4));
             const int cc = k % (2 * HS / 4);
             c = cc < HS / 4 ? -HS + 4 * cc : TZ + 4 * (cc - HS / 4);
         }
@@ -707,7 +757,7 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
         // faster than 4 at c2, batch 16: less code in the hot loop)
         constexpr int P2R = 2;
 #pragma unroll 1
-        for (int q0 = 0; q0 < 4; q0 += P2R) {
+        for (int q0 = 0; q0 < G::RS; q0 += P2R) {
         // the model's operands first: their latency runs under the derivatives
         float4 vp2r[P2R], vs2r[P2R];
 #pragma unroll
@@ -855,7 +905,7 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
 
     // ---- phase 3: U-stage on the tile's own cells (2 rows x 4 columns) ------
     {
-        const int rr = 2 * (tid / (TZ / 4));
+        const int rr = G::RU * (tid / (TZ / 4));
         const int c = 4 * (tid % (TZ / 4));
         const int scol = c + HS;
         const float dt = p.dt;
@@ -873,9 +923,9 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
         //  - U boxes too small for the above (N = 2): one row per pass.
         // Measured at c2, batch 16: forward -1.9 %, receiver -3.0 %,
         // reconstruction -2.0 % against one row per pass.
-        constexpr bool kShare3 = MODE == kFwd && G::UR * G::UC >= TX * TZ + 12 * kThreads;
-        constexpr bool kShare4 = MODE == kRcv && G::UR * G::UC >= 16 * kThreads;
-        constexpr bool kCarry = MODE == kRec;
+        constexpr bool kShare3 = G::RU == 2 && MODE == kFwd && G::UR * G::UC >= TX * TZ + 12 * kThreads;
+        constexpr bool kShare4 = G::RU == 2 && MODE == kRcv && G::UR * G::UC >= 16 * kThreads;
+        constexpr bool kCarry = G::RU == 2 && MODE == kRec;
         float4* const c3x = reinterpret_cast<float4*>(sUx + TX * TZ) + tid;
         float4* const c3z = reinterpret_cast<float4*>(sUz + TX * TZ) + tid;
         float4* const c4x = reinterpret_cast<float4*>(sUx) + tid;
@@ -899,7 +949,7 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
         // a rolled two-iteration loop: half the code of an unrolled pair of
         // rows, which keeps the hot path inside the instruction cache
 #pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < G::RU; ++q) {
             const int r = rr + q;
             const int gi = x0 + r;
             const int g = gi * P + (z0 + c);
@@ -1094,18 +1144,18 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
     return true;
 }
 
-template <int N, int MODE>
-__global__ void __launch_bounds__(kThreads, 2) k_step(const __grid_constant__ StepArgs p) {
-    extern __shared__ __align__(128) float4 smem4[];
-    float* sm = reinterpret_cast<float*>(smem4);
-    using G = TileGeo<N>;
-    const int tz = blockIdx.x % p.tiles_z, tx = blockIdx.x / p.tiles_z;
+// One CTA of a step launch: tile `tile` of shot blockIdx.y.
+template <int N, int MODE, class G>
+__device__ __forceinline__ void step_cta(const StepArgs& p, int tile, float* sm) {
+    const int tz = tile % p.tiles_z, tx = tile / p.tiles_z;
     const int x0 = p.tile_x0 + tx * G::TX, z0 = p.tile_z0 + tz * G::TZ;
     if (MODE != kRec && x0 >= p.X - N) {
         // every row of the tile lies outside the update domain [N, X-N) of
         // the forward and receiver steps: its cells are never written (they
         // were zeroed with the shot's state), so only the forward's record
         // samples of these rows, zeros, are stored (PS:307-311 records every x)
+        pdl_launch_dependents();
+        pdl_wait();
         if (MODE == kFwd && p.record) {
             const ShotDesc& d = p.shots[blockIdx.y];
             if (d.rz >= z0 && d.rz < z0 + G::TZ)
@@ -1120,10 +1170,11 @@ __global__ void __launch_bounds__(kThreads, 2) k_step(const __grid_constant__ St
     if (threadIdx.x == 0) {   // the tile's copies first: they overlap everything up to phase 1
         mbar_init(&bar, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-        issue_u_box<N>(p, sm, x0, z0, blockIdx.y, &bar);
+        pdl_wait();
+        issue_u_box<G>(p, sm, x0, z0, blockIdx.y, &bar);
     }
     const ShotDesc& d = p.shots[blockIdx.y];
-    if ((int)blockIdx.x >= (MODE == kRec ? d.rec_tiles_x : d.tiles_x) * p.tiles_z) {
+    if (tx * G::TX >= (MODE == kRec ? d.X - 2 * p.L : d.X)) {
         // beyond this shot's width (per-shot sub-grids): the copies (of cells
         // outside the shot's grid) land before the shared memory is released
         if (threadIdx.x == 0) mbar_wait(&bar, 0u);
@@ -1131,11 +1182,18 @@ __global__ void __launch_bounds__(kThreads, 2) k_step(const __grid_constant__ St
     }
     const Geo gm = geo_of(d);
     const ShotView sv = shot_view(p, blockIdx.y);
-    const TileFlags f = tile_flags<N, MODE>(p, gm, sv, x0, z0);
-    prefetch_tile<N, MODE>(p, gm, x0, z0, blockIdx.y, f);
-    if (MODE == kRec && f.ring) prefetch_ring<N>(p, gm, d, x0, z0);
+    const TileFlags f = tile_flags<G, MODE>(p, gm, sv, x0, z0);
+    if (!G::mid) prefetch_tile<G, MODE>(p, gm, x0, z0, blockIdx.y, f);
+    if (MODE == kRec && f.ring) prefetch_ring<G>(p, gm, d, x0, z0);
     __syncthreads();   // the mbarrier is initialised
-    step_tile<N, MODE>(p, gm, sv, sm, x0, z0, f, &bar, 0u);
+    pdl_wait();
+    step_tile<G, MODE>(p, gm, sv, sm, x0, z0, f, &bar, 0u);
+}
+
+template <int N, int MODE, class G = TileGeo<N>>
+__global__ void __launch_bounds__(kThreads, 2) k_step(const __grid_constant__ StepArgs p) {
+    extern __shared__ __align__(128) float4 smem4[];
+    step_cta<N, MODE, G>(p, blockIdx.x, reinterpret_cast<float*>(smem4));
 }
 
 // The same step as a persistent launch with a dynamic work queue: a few
@@ -1175,13 +1233,13 @@ __global__ void __launch_bounds__(kThreads, 2) k_step_q(const __grid_constant__ 
         const ShotDesc& d = p.shots[b];
         if (tx < (MODE == kRec ? d.rec_tiles_x : d.tiles_x)) {   // within this shot's width
             const int x0 = p.tile_x0 + tx * G::TX, z0 = p.tile_z0 + tz * G::TZ;
-            if (threadIdx.x == 0) issue_u_box<N>(p, sm, x0, z0, b, &bar);
+            if (threadIdx.x == 0) issue_u_box<G>(p, sm, x0, z0, b, &bar);
             const Geo gm = geo_of(d);
             const ShotView sv = shot_view(p, b);
-            const TileFlags f = tile_flags<N, MODE>(p, gm, sv, x0, z0);
-            prefetch_tile<N, MODE>(p, gm, x0, z0, b, f);
-            if (MODE == kRec && f.ring) prefetch_ring<N>(p, gm, d, x0, z0);
-            if (!step_tile<N, MODE>(p, gm, sv, sm, x0, z0, f, &bar, parity)) break;   // uniform: reported
+            const TileFlags f = tile_flags<G, MODE>(p, gm, sv, x0, z0);
+            prefetch_tile<G, MODE>(p, gm, x0, z0, b, f);
+            if (MODE == kRec && f.ring) prefetch_ring<G>(p, gm, d, x0, z0);
+            if (!step_tile<G, MODE>(p, gm, sv, sm, x0, z0, f, &bar, parity)) break;   // uniform: reported
             parity ^= 1u;
         }
         __syncthreads();   // the tile's shared memory is free and the next index is visible

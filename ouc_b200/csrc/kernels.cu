@@ -6,33 +6,38 @@
 #include <algorithm>
 
 #include "fd_march.cuh"
+#include "fd_small.cuh"
 #include "fd_step.cuh"
 #include "ouc_internal.h"
 
 namespace ouc {
 
+template <class K>
+static cudaError_t configure_kernel(K kernel, int bytes) {
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    if (e == cudaSuccess)
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared);
+    return e;
+}
+
 template <int N, int MODE>
 static cudaError_t configure_one() {
-    cudaError_t e = cudaFuncSetAttribute(k_step<N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TileGeo<N>::bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_step<N, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_step_q<N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, TileGeo<N>::bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_step_q<N, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_march<N, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MarchGeo<N>::bytes);
-    if (e == cudaSuccess)
-        e = cudaFuncSetAttribute(k_march<N, MODE>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                 cudaSharedmemCarveoutMaxShared);
+    cudaError_t e = configure_kernel(k_step<N, MODE>, TileGeo<N>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_step<N, MODE, MidGeo<N>>, MidGeo<N>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_small<N, MODE, 16, 1>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_small<N, MODE, 16, 2>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_small<N, MODE, 24, 1>, SmallGeo<N, 24>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_step_q<N, MODE>, TileGeo<N>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_march<N, MODE>, MarchGeo<N>::bytes);
     return e;
 }
 
 template <int N>
 static cudaError_t configure_modes() {
-    cudaError_t e = configure_one<N, kFwd>();
+    cudaError_t e = configure_kernel(k_small_back<N, 16, 1>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_small_back<N, 16, 2>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = configure_kernel(k_small_back<N, 24, 1>, SmallGeo<N, 24>::bytes);
+    if (e == cudaSuccess) e = configure_one<N, kFwd>();
     if (e == cudaSuccess) e = configure_one<N, kRcv>();
     if (e == cudaSuccess) e = configure_one<N, kRec>();
     return e;
@@ -55,6 +60,73 @@ int march_segments(Mode mode, const StepArgs& a) {
     return (row_end - row0 + a.seg_rows - 1) / a.seg_rows;
 }
 
+// Launch with programmatic stream serialization: the kernel may start before
+// the launch ahead of it in the stream has finished (pdl_wait orders them).
+template <class... P, class... A>
+static void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, args...);
+}
+
+struct Grid {
+    int tiles_z, tiles;
+};
+static Grid grid_of(Mode mode, const StepArgs& a, int TX, int TZ) {
+    const int rows = mode == kRec ? a.X - 2 * a.L : a.X, cols = mode == kRec ? a.Z - a.L - a.tile_z0 : a.Z;
+    Grid g;
+    g.tiles_z = (cols + TZ - 1) / TZ;
+    g.tiles = (rows + TX - 1) / TX * g.tiles_z;
+    return g;
+}
+// 24-row tiles may end beyond the rows the field allocation keeps for 32-row ones.
+static bool fits24(Mode mode, const StepArgs& a, int N) {
+    const int rows = mode == kRec ? a.X - 2 * a.L : a.X, x0 = mode == kRec ? a.tile_x0 : 0;
+    return x0 + (rows + 23) / 24 * 24 + N <= (int)(a.fstride / a.pitch) - kGX;
+}
+// Tile shape of a launch, or of two that run beside each other.  A launch
+// lasts as long as its waves of CTAs, so what decides is how many tiles there
+// are for the SMs.  us per forward step without strips / per back-step, one
+// shot unless stated, B200, half-order 5 (6 where marked):
+//     grid (padded)      small 16x1   small 24   small 16x2   mid    large
+//     160 x 120 (6)        6.7          9.0         9.9       10.9    19.3
+//     296 x 296           11.6          8.3         9.9       12.9    23.4
+//     397 x 301 (6)       12.9         15.9        11.5       13.5    24.2
+//     560 x 310 back      26.6         24.2        22.1       19.0    29.3
+//     1060 x 560          44.0          -          35.1       24.1    28.9
+//     1060 x 560, 2 shots 95.7         87.7        71.7       43.0    46.5
+//     1060 x 560, 4 shots  -            -            -        84.5    82.3
+// Small tiles in one wave: one CTA of 576 threads per SM (16 rows) or of 768
+// (24 rows); two of 576 with fewer registers each up to two per SM.  Beyond
+// that 16 x 64 tiles, whose last wave is half as long as a 32 x 64 one, until
+// the launch has about five waves of them; then the 32 x 64 tiles, which
+// recompute less halo.
+Tier pick_tier(int N, const StepArgs* rec, const StepArgs* other, Mode other_mode, int nshots) {
+    int t16 = 0, t24 = 0, mid = 0;
+    bool ok24 = true;
+    auto add = [&](Mode mode, const StepArgs& a) {
+        t16 += grid_of(mode, a, 16, 32).tiles * nshots;
+        t24 += grid_of(mode, a, 24, 32).tiles * nshots;
+        mid += grid_of(mode, a, 16, 64).tiles * nshots;
+        ok24 = ok24 && fits24(mode, a, N);
+    };
+    if (rec) add(kRec, *rec);
+    if (other) add(other_mode, *other);
+    const int set = (other ? other : rec)->nsm, nsm = set > 0 ? set : 148;
+    if (t16 <= nsm) return kSmall16;
+    if (t24 <= nsm && ok24) return kSmall24;
+    if (t16 <= 2 * nsm) return kSmall16x2;
+    return mid <= 10 * nsm ? kMid : kLarge;
+}
+
 template <int N, int MODE>
 static void launch_one(const StepArgs& a, int tiles_x, int nshots, cudaStream_t s) {
     if (a.seg_rows > 0) {
@@ -68,8 +140,39 @@ static void launch_one(const StepArgs& a, int tiles_x, int nshots, cudaStream_t 
         k_step_q<N, MODE><<<grid, kThreads, TileGeo<N>::bytes, s>>>(a, nshots, ntiles);
         return;
     }
-    constexpr int bytes = TileGeo<N>::bytes;
-    k_step<N, MODE><<<dim3(tiles_x * a.tiles_z, nshots), kThreads, bytes, s>>>(a);
+    const Mode mode = (Mode)MODE;
+    const Tier tier = a.tier != kAuto ? (Tier)a.tier : pick_tier(N, nullptr, &a, mode, nshots);
+    if (tier == kLarge) {
+        launch_pdl(k_step<N, MODE>, dim3(tiles_x * a.tiles_z, nshots), kThreads, TileGeo<N>::bytes, s, a);
+        return;
+    }
+    StepArgs b = a;
+    if (tier == kMid) {
+        const Grid g = grid_of(mode, a, 16, 64);
+        launch_pdl(k_step<N, MODE, MidGeo<N>>, dim3(g.tiles, nshots), kThreads, MidGeo<N>::bytes, s, b);
+        return;
+    }
+    const Grid g = grid_of(mode, a, tier == kSmall24 ? 24 : 16, 32);
+    const dim3 grid(g.tiles, nshots);
+    b.tiles_z = g.tiles_z;
+    if (tier == kSmall24) launch_pdl(k_small<N, MODE, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, b);
+    else if (tier == kSmall16) launch_pdl(k_small<N, MODE, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, b);
+    else launch_pdl(k_small<N, MODE, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, b);
+}
+
+template <int N>
+static int launch_back_n(const StepArgs& rec, const StepArgs& rcv, Tier tier, int nshots, cudaStream_t s) {
+    const int tx = tier == kSmall24 ? 24 : 16;
+    const Grid g0 = grid_of(kRec, rec, tx, 32), g1 = grid_of(kRcv, rcv, tx, 32);
+    StepArgs a0 = rec, a1 = rcv;
+    a0.tiles_z = g0.tiles_z;
+    a1.tiles_z = g1.tiles_z;
+    const dim3 grid(g0.tiles + g1.tiles, nshots);
+    if (tier == kSmall24) launch_pdl(k_small_back<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, a0, a1, g0.tiles);
+    else if (tier == kSmall16) launch_pdl(k_small_back<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a0, a1, g0.tiles);
+    else if (tier == kSmall16x2) launch_pdl(k_small_back<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a0, a1, g0.tiles);
+    else return 1;
+    return 0;
 }
 
 template <int N>
@@ -85,9 +188,9 @@ static int launch_mode(Mode m, const StepArgs& a, int tiles_x, int nshots, cudaS
 // Refuses (returns 1) a launch whose state map is missing or whose now[]
 // pointers are not fields of the mapped block, so that no step kernel runs
 // a tensor copy with coordinates the map does not describe.
-int launch_step(int N, Mode mode, const StepArgs& a, int tiles_x, int nshots, cudaStream_t s) {
+static int resolve_fields(const StepArgs& a, StepArgs& b) {
     if (!a.state0 || a.fstride == 0 || a.nfields <= 0) return 1;
-    StepArgs b = a;
+    b = a;
     const float* f0 = a.state0 + (size_t)kGX * a.pitch + kZOFF;   // field 0 of slot 0, cell (0, 0)
     auto field_of = [&](const float* q) -> int {
         if (!q || q < f0) return -1;
@@ -103,10 +206,30 @@ int launch_step(int N, Mode mode, const StepArgs& a, int tiles_x, int nshots, cu
         b.fold_field[q] = field_of(a.f_old[q]);
     }
     for (int q = 0; q < 8; ++q) b.o_field[q] = field_of(a.o[q]);
+    return 0;
+}
+
+int launch_step(int N, Mode mode, const StepArgs& a, int tiles_x, int nshots, cudaStream_t s) {
+    StepArgs b;
+    if (resolve_fields(a, b)) return 1;
     switch (N) {
         case 2: return launch_mode<2>(mode, b, tiles_x, nshots, s);
         case 5: return launch_mode<5>(mode, b, tiles_x, nshots, s);
         case 6: return launch_mode<6>(mode, b, tiles_x, nshots, s);
+    }
+    return 1;
+}
+
+// The reconstruction + imaging of one back-step and the receiver step after
+// it as one launch of small tiles.  Refuses as launch_step does, and any
+// other tile shape.
+int launch_back(int N, const StepArgs& rec, const StepArgs& rcv, int nshots, cudaStream_t s) {
+    StepArgs b0, b1;
+    if (resolve_fields(rec, b0) || resolve_fields(rcv, b1)) return 1;
+    switch (N) {
+        case 2: return launch_back_n<2>(b0, b1, (Tier)rcv.tier, nshots, s);
+        case 5: return launch_back_n<5>(b0, b1, (Tier)rcv.tier, nshots, s);
+        case 6: return launch_back_n<6>(b0, b1, (Tier)rcv.tier, nshots, s);
     }
     return 1;
 }
@@ -154,6 +277,16 @@ cudaError_t encode_for(StepArgs& a, const float* state0, int pitch, int rows, in
                             sbox, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r3 != CUDA_SUCCESS) return cudaErrorInvalidValue;
+    auto u_box = [&](CUtensorMap* m, int uc, int ur) {
+        const cuuint32_t ubox[4] = {(cuuint32_t)uc, (cuuint32_t)ur, 1, 1};
+        return enc(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(state0), dims, strides, ubox, estr,
+                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+    };
+    if (!u_box(&a.mid_map, MidGeo<N>::UC, MidGeo<N>::UR) ||
+        !u_box(&a.small_map[0], SmallGeo<N, 16>::UC, SmallGeo<N, 16>::UR) ||
+        !u_box(&a.small_map[1], SmallGeo<N, 24>::UC, SmallGeo<N, 24>::UR))
+        return cudaErrorInvalidValue;
     a.state0 = state0;
     a.fstride = fstride;
     a.nfields = nfields;

@@ -67,6 +67,10 @@ inline constexpr double kStencilWeights[7][6] = {
 };
 
 enum Mode : int { kFwd = 0, kRcv = 1, kRec = 2 };
+// Tile shape of a step launch (pick_tier): 32 x 64 or 16 x 64 cells (fd_step.cuh),
+// or the small tiles of fd_small.cuh, 24 or 16 rows by 32 columns, the last
+// with two CTAs per SM or one.
+enum Tier : int { kAuto = 0, kLarge, kMid, kSmall24, kSmall16x2, kSmall16 };
 
 // Boundary ring: the cells within N of the interior edge, on both sides
 // (the reference's four strips of 2N rows/columns, PS:1230-1287, trimmed to
@@ -157,6 +161,8 @@ struct StepArgs {
     alignas(64) CUtensorMap box_map;
     alignas(64) CUtensorMap own_map;     // the same block, box = one tile's own cells (TZ x TX): L2 prefetches
     alignas(64) CUtensorMap s_map;       // the same block, box = one tile's S region (SC x SR): L2 prefetches
+    alignas(64) CUtensorMap mid_map;     // the same block, box = the U box of a 16 x 64 tile (MidGeo)
+    alignas(64) CUtensorMap small_map[2];   // the same block, box = the U box of a small tile of 16, 24 rows (SmallGeo)
     const float* state0;
     size_t fstride;                   // floats per field of the block
     int nfields;                      // fields per shot slot of the block
@@ -174,6 +180,7 @@ struct StepArgs {
     int strip_prec;                   // StripPrec of the strips
     int comp_image;                   // kRec: compensated (Kahan) imaging sums, comp[] below
     int density;                      // variable density: scale the U-stage by the buoyancy
+    int tier;                         // Tier of the launch; kAuto: chosen for it alone
     int seg_rows;                     // > 0: the x-marching kernel, segments of this many rows (a multiple of 16);
                                       // 0: one CTA per 32 x 64 tile; -1: the tile kernel with a dynamic queue
     int nsm;                          // SMs of the device (persistent grid of the queue form)
@@ -274,6 +281,9 @@ struct GradStackArgs {
 cudaError_t encode_box_map(StepArgs& a, const float* state0, int pitch, int rows, int nfields, int nslots,
                            size_t fstride, int N);
 int launch_step(int N, Mode mode, const StepArgs& a, int tiles_x, int nshots, cudaStream_t s);
+// Tile shape of a launch of `mode`, run beside a reconstruction launch when rec is given.
+Tier pick_tier(int N, const StepArgs* rec, const StepArgs* other, Mode mode, int nshots);
+int launch_back(int N, const StepArgs& rec, const StepArgs& rcv, int nshots, cudaStream_t s);
 // Segments of the x-marching kernel for a launch (rows of the widest shot).
 int march_segments(Mode mode, const StepArgs& a);
 cudaError_t configure_step_kernels(int N);
