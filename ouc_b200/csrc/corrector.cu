@@ -1,26 +1,28 @@
 // Learned dispersion corrector (include/ouc_corrector.h): a 4-layer 5x5 CNN
 // whose convolutions run as implicit GEMMs on the sm_100a tensor cores.
 //
-// One convolution tile = 128 consecutive pixels of one image row (GEMM M),
-// all output channels (N = 32 or 16), K = 25 taps x input channels.  The CTA
-// stages the 5-row x 132-column input patch in shared memory in the
-// no-swizzle K-major "core matrix" layout -- [row][channel chunk of 8][column]
-// [8 channels], 16 bytes per (column, chunk) -- so that the A operand of tap
-// (dx, dz) is simply the patch shifted by (dx, dz): a shared-memory matrix
-// descriptor whose start address moves by 16 * (dx * chunks * 132 + dz)
+// A convolution's GEMM M is 128 consecutive pixels of one image row, N all
+// output channels (32 or 16), K 25 taps x input channels.  A work item is RB
+// consecutive rows of 128 pixels; its (RB + 4)-row x 132-column input patch
+// (zeros outside the image) lies in shared memory in the no-swizzle K-major "core matrix" layout -- [row][channel chunk of 8]
+// [column][8 channels], 16 bytes per (column, chunk) -- so that the A operand
+// of tap (dx, dz) is simply the patch shifted by (dx, dz): a shared-memory
+// matrix descriptor whose start address moves by 16 * (dx * chunks * 132 + dz)
 // bytes, with the leading-dimension offset = one chunk plane (132 * 16 B)
 // and the stride offset = 8 pixels (128 B).  No im2col copy is made.  The
 // weights of all taps sit in shared memory for the whole (persistent) CTA in
-// the same layout, [tap][chunk][out channel][8].  One thread issues the
-// 25 * (channels / 16) tcgen05.mma instructions (kind::f16, BF16 x BF16 ->
-// FP32 in tensor memory), commits them to an mbarrier, and the four warps
-// read the 128 x N accumulator back with tcgen05.ld (warp w owns lanes
-// 32w..32w+31, i.e. pixels 32w..32w+31) for the epilogue: bias + ReLU ->
-// BF16 activations, bias -> FP32 outputs, or (input-gradient pass) the ReLU
-// mask of the forward activation.
+// the same layout, [tap][chunk][out channel][8].  The roles are split over
+// warps and the items pipelined two deep: eight warps copy (16-byte
+// asynchronous copies; tensor copies of this layout, whose innermost extent
+// is 16 bytes, were no faster), one thread issues the 25 * (channels / 16) tcgen05.mma instructions per row (kind::f16,
+// BF16 x BF16 -> FP32 in tensor memory), and four warps read the finished
+// 128 x N accumulators back with tcgen05.ld (warp w owns lanes 32w..32w+31,
+// i.e. pixels 32w..32w+31) for the epilogue: bias + ReLU -> BF16 activations,
+// bias -> FP32 outputs, or (input-gradient pass) the ReLU mask of the forward
+// activation.
 //
-// Every wait is bounded: an mbarrier that does not complete within ~2 s of
-// polling sets the network's error flag; the CTA then waits once more (also
+// Every wait is bounded: an mbarrier that does not complete within ~2 s
+// sets the network's error flag; the CTA then waits once more (also
 // bounded) and releases its tensor memory.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -45,9 +47,11 @@ constexpr int kTile = 128;            // GEMM M: pixels per tile
 constexpr int kPC = kTile + 4;        // patch columns (2 + 2 halo)
 constexpr int kTaps = 25;
 constexpr int kMaxPairs = 32 * 32;     // (cin, cout) pairs of the widest layer
-constexpr int kMaxRowBlocks = 64;      // CTAs (partial-sum slots) of k_wgrad_tc
-constexpr int kBgradBlocks = 256;      // blocks of k_bgrad (8 warps each)
-constexpr int kThreadsConv = 128;
+constexpr int kRB = 2;                 // image rows of a work item
+constexpr int kWgradCtas = 148;        // CTAs (partial-sum slots) of k_wgrad_tc
+constexpr int kBgradBlocks = 592;      // blocks of k_bgrad
+constexpr int kCopyThreads = 256;      // copy warps 5-12
+constexpr int kThreadsConv = 160 + kCopyThreads;   // epilogue warps 0-3, MMA warp 4, copy warps
 
 struct LayerDims {
     int cin, cout, cin_pad, cout_pad;
@@ -100,27 +104,37 @@ __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
 }
 
-__device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
+// One hardware-suspended try: the thread sleeps until the phase completes or
+// a time limit of about 0.1 ms passes (no busy polling beside the copies).
+__device__ __forceinline__ bool mbar_try(uint64_t* bar, uint32_t parity) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred P1;\n\t"
-        "mbarrier.test_wait.parity.shared::cta.b64 P1, [%1], %2;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 P1, [%1], %2, %3;\n\t"
         "selp.b32 %0, 1, 0, P1;\n\t}\n"
         : "=r"(done)
-        : "r"(smem_u32(bar)), "r"(parity)
+        : "r"(smem_u32(bar)), "r"(parity), "r"(100000u)
         : "memory");
     return done != 0;
 }
 
-// Poll with back-off; false after ~2^24 polls (well over a second).
+// Bounded wait: false after 2^14 suspended tries (over a second).
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 24); ++i) {
-        if (mbar_test(bar, parity)) return true;
-        if (i > 64) __nanosleep(64);
-    }
+    for (int i = 0; i < (1 << 14); ++i)
+        if (mbar_try(bar, parity)) return true;
     return false;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t* bar) {
+    asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+// 16-byte asynchronous copy, zero-filled when !in (src is then not read).
+__device__ __forceinline__ void cp16(uint32_t dst, const void* src, bool in) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16u : 0u) : "memory");
+}
+__device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
@@ -181,121 +195,199 @@ struct ConvArgs {
     int* err;
 };
 
+// Work items of kRB rows x 128 pixels.
+struct Items {
+    int tiles_w, row_blocks, count;
+    __host__ __device__ Items(int n, int H, int W)
+        : tiles_w((W + kTile - 1) / kTile), row_blocks((H + kRB - 1) / kRB), count(n * row_blocks * tiles_w) {}
+    __device__ __forceinline__ void at(int item, int& img, int& h, int& z0) const {
+        const int tw = item % tiles_w, rest = item / tiles_w;
+        img = rest / row_blocks;
+        h = (rest - img * row_blocks) * kRB;
+        z0 = tw * kTile;
+    }
+};
+
+// This thread's copies have landed: make them visible to the tensor core's
+// proxy and count the thread in.
+__device__ __forceinline__ void hand_over(uint64_t* full) {
+    cp_wait<0>();
+    fence_proxy_async();
+    mbar_arrive(full);
+}
+
+// Copy threads (t = 0 .. kCopyThreads-1): rows h .. h+ROWS-1, columns
+// z .. z+COLS-1 of one NHWC image with C channels into shared memory as
+// [row][chunk of 8][column][8 channels], zeros outside the image.  A thread
+// keeps its chunk and column and walks down the rows.
+template <int C, int ROWS, int COLS>
+__device__ __forceinline__ void copy_patch(uint32_t dst, const bf16* x, int img, int h, int z, int H, int W, int t) {
+    constexpr int NQ = C / 8, CPP = kCopyThreads / NQ;   // columns per pass
+    const int q = t % NQ, c0 = t / NQ;
+    const ptrdiff_t row = (ptrdiff_t)W * C;
+#pragma unroll
+    for (int p = 0; p < (COLS + CPP - 1) / CPP; ++p) {
+        const int c = c0 + p * CPP, gz = z + c;
+        if (c >= COLS) break;
+        const bool col = gz >= 0 && gz < W;
+        const bf16* src = x + (((ptrdiff_t)img * H + h) * W + gz) * C + q * 8;
+        const uint32_t d = dst + (q * COLS + c) * 16;
+#pragma unroll
+        for (int r = 0; r < ROWS; ++r) {
+            const bool in = col && (unsigned)(h + r) < (unsigned)H;
+            cp16(d + r * NQ * COLS * 16, in ? src + r * row : x, in);
+        }
+    }
+}
+
 template <int CIN, int COUT>
 struct ConvGeo {
     static constexpr int NQ = CIN / 8;
     static constexpr int w_bytes = kTaps * CIN * COUT * 2;
-    static constexpr int p_bytes = 5 * NQ * kPC * 16;
-    static constexpr int bytes = w_bytes + p_bytes;
+    static constexpr int row_bytes = NQ * kPC * 16;
+    static constexpr int p_bytes = (kRB + 4) * row_bytes;     // one stage
+    static constexpr int bytes = w_bytes + 2 * p_bytes;
+    static constexpr int acc_cols = 2 * kRB * COUT;
+    static constexpr int tmem_cols = acc_cols <= 32 ? 32 : acc_cols <= 64 ? 64 : acc_cols <= 128 ? 128 : 256;
+    static_assert(acc_cols <= 256, "two accumulator stages fit tensor memory");
+    static_assert(w_bytes % 128 == 0 && row_bytes % 128 == 0, "tensor-copy destinations are 128-byte aligned");
 };
 
+// Bound: the MMAs, about 85 cycles each whatever their 16 or 32 columns (the
+// same with the copies left out).  A 32 -> 32 layer on 4 images of 290 x 158:
+// 72 -> 33 us (first form: 128 threads
+// staged the patch of one row, then waited for its MMAs).
 template <int CIN, int COUT, int EPI>
-__global__ void __launch_bounds__(kThreadsConv) k_conv5(const ConvArgs a) {
+__global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
     using G = ConvGeo<CIN, COUT>;
     constexpr int NQ = G::NQ;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* s_w = smem;
     uint8_t* s_p = smem + G::w_bytes;
-    __shared__ __align__(8) uint64_t bar;
+    __shared__ __align__(8) uint64_t full[2], done[2], drained[2];   // copied; multiplied; accumulators read
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const Items items(a.n, a.H, a.W);
 
-    for (int i = tid; i < G::w_bytes / 16; i += kThreadsConv)
-        reinterpret_cast<uint4*>(s_w)[i] = reinterpret_cast<const uint4*>(a.w)[i];
-    if (tid == 0) mbar_init(&bar, 1);
+    if (tid == 0) {
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&full[s], kCopyThreads);
+            mbar_init(&done[s], 1);
+            mbar_init(&drained[s], 128);
+        }
+    }
+    for (int i = tid; i < G::w_bytes / 16; i += kThreadsConv) cp16(smem_u32(s_w) + i * 16, a.w + i * 8, true);
+    cp_commit();
+    cp_wait<0>();
+    fence_proxy_async();
     __syncwarp();   // .sync.aligned tcgen05 instructions need a converged warp
-    if (warp == 0) tmem_alloc(&tmem_base, 32);
+    if (warp == 0) tmem_alloc(&tmem_base, G::tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const int tiles_w = (a.W + kTile - 1) / kTile;
-    const int ntiles = a.n * a.H * tiles_w;
-    uint32_t phase = 0;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int tw = tile % tiles_w, row = tile / tiles_w;
-        const int img = row / a.H, h = row - img * a.H;
-        const int z0 = tw * kTile;
-        // input patch: rows h-2..h+2, columns z0-2..z0+129, zero outside the image
-        for (int i = tid; i < 5 * kPC * NQ; i += kThreadsConv) {
-            const int q = i % NQ, rest = i / NQ, c = rest % kPC, r = rest / kPC;
-            const int gh = h + r - 2, gz = z0 + c - 2;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gh >= 0 && gh < a.H && gz >= 0 && gz < a.W)
-                v = *reinterpret_cast<const uint4*>(a.x + (((size_t)img * a.H + gh) * a.W + gz) * CIN + q * 8);
-            *reinterpret_cast<uint4*>(s_p + ((size_t)(r * NQ + q) * kPC + c) * 16) = v;
+    bool ok = true;
+    if (warp >= 5) {   // copies: a stage is free once the MMAs of the item two before are done
+        int k = 0;
+        for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
+            const int s = k & 1;
+            if (k > 0) hand_over(&full[s ^ 1]);
+            if (k >= 2 && !(ok = mbar_wait(&done[s], (uint32_t)((k >> 1) - 1) & 1u))) break;
+            int img, h, z0;
+            items.at(it, img, h, z0);
+            copy_patch<CIN, kRB + 4, kPC>(smem_u32(s_p) + s * G::p_bytes, a.x, img, h - 2, z0 - 2, a.H, a.W, tid - 160);
+            cp_commit();
         }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
-            const uint32_t pb = smem_u32(s_p), wb = smem_u32(s_w);
-            constexpr uint32_t idesc = idesc_bf16(kTile, COUT);
-            uint32_t acc = 0;
+        if (k > 0 && ok) hand_over(&full[(k - 1) & 1]);
+    } else if (tid == 128) {   // MMAs
+        const uint64_t bd0 = umma_desc(smem_u32(s_w), COUT * 16, 128);
+        constexpr uint32_t idesc = idesc_bf16(kTile, COUT);
+        int k = 0;
+        for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
+            const int s = k & 1;
+            const uint32_t ph = (uint32_t)(k >> 1) & 1u;
+            ok = (k < 2 || mbar_wait(&drained[s], ph ^ 1u)) && mbar_wait(&full[s], ph);
+            if (!ok) break;
+            tc_fence_after();
+            // descriptors: the start address (in 16-byte units) is the low
+            // field, so a tap or chunk is one addition
+            const uint64_t ad0 = umma_desc(smem_u32(s_p) + s * G::p_bytes, kPC * 16, 128);
 #pragma unroll 1
-            for (int dx = 0; dx < 5; ++dx) {
-#pragma unroll 1
-                for (int dz = 0; dz < 5; ++dz) {
+            for (int r = 0; r < kRB; ++r) {
+                const uint32_t d = tmem + (uint32_t)((s * kRB + r) * COUT);
 #pragma unroll
-                    for (int ks = 0; ks < NQ / 2; ++ks) {
-                        const uint32_t tap = dx * 5 + dz;
-                        const uint64_t ad = umma_desc(pb + ((dx * NQ + 2 * ks) * kPC + dz) * 16, kPC * 16, 128);
-                        const uint64_t bd = umma_desc(wb + ((tap * NQ + 2 * ks) * COUT) * 16, COUT * 16, 128);
-                        umma_bf16(tmem, ad, bd, idesc, acc);
-                        acc = 1;
+                for (int dx = 0; dx < 5; ++dx) {
+                    const uint64_t adr = ad0 + (uint32_t)((r + dx) * NQ * kPC);
+#pragma unroll
+                    for (int dz = 0; dz < 5; ++dz) {
+#pragma unroll
+                        for (int ks = 0; ks < NQ / 2; ++ks) {
+                            const int tap = dx * 5 + dz;
+                            umma_bf16(d, adr + (uint32_t)(2 * ks * kPC + dz), bd0 + (uint32_t)((tap * NQ + 2 * ks) * COUT), idesc,
+                                      tap || ks ? 1u : 0u);
+                        }
                     }
                 }
             }
-            umma_commit(&bar);
+            umma_commit(&done[s]);
         }
-        const bool done = mbar_wait(&bar, phase);
-        phase ^= 1u;
-        if (!__syncthreads_and(done)) {
-            if (tid == 0) atomicExch(a.err, 1);
-            mbar_wait(&bar, phase ^ 1u);   // one more bounded wait for the MMAs in flight
-            break;
-        }
-        tc_fence_after();
-        uint32_t r[COUT];
-        __syncwarp();
-        tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16), r);
-        const int gz = z0 + warp * 32 + lane;
-        if (gz < a.W) {
-            const size_t p = ((size_t)img * a.H + h) * a.W + gz;
-            if (EPI == kOut) {
-                float* y = static_cast<float*>(a.y) + p * a.cout_real;
+        // the last commits complete before the tensor memory is freed
+        for (int q = k - 2 > 0 ? k - 2 : 0; q < k; ++q) ok = mbar_wait(&done[q & 1], (uint32_t)(q >> 1) & 1u) && ok;
+    } else if (warp < 4) {   // epilogue
+        int k = 0;
+        for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
+            const int s = k & 1;
+            ok = __all_sync(0xffffffffu, mbar_wait(&done[s], (uint32_t)(k >> 1) & 1u));
+            if (!ok) break;
+            tc_fence_after();
+            uint32_t r[kRB][COUT];
 #pragma unroll
-                for (int c = 0; c < COUT; ++c)
-                    if (c < a.cout_real) y[c] = __uint_as_float(r[c]) + a.bias[c];
-            } else {
-                uint4* y = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + p * COUT);
-                const uint4* mk = EPI == kDgrad ? reinterpret_cast<const uint4*>(a.mask + p * COUT) : nullptr;
+            for (int q = 0; q < kRB; ++q)
+                tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((s * kRB + q) * COUT), r[q]);
+            tc_fence_before();
+            mbar_arrive(&drained[s]);
+            int img, h, z0;
+            items.at(it, img, h, z0);
+            const int gz = z0 + warp * 32 + lane;
+            if (gz >= a.W) continue;
 #pragma unroll
-                for (int c8 = 0; c8 < COUT / 8; ++c8) {
-                    __align__(16) bf16 o[8];
-                    __align__(16) bf16 mv[8];
-                    if (EPI == kDgrad) *reinterpret_cast<uint4*>(mv) = mk[c8];
+            for (int q = 0; q < kRB; ++q) {
+                if (h + q >= a.H) break;
+                const size_t p = ((size_t)img * a.H + h + q) * a.W + gz;
+                if (EPI == kOut) {
+                    float* y = static_cast<float*>(a.y) + p * a.cout_real;
 #pragma unroll
-                    for (int k = 0; k < 8; ++k) {
-                        const int c = 8 * c8 + k;
-                        float v = __uint_as_float(r[c]);
-                        if (EPI == kHidden) v = fmaxf(v + a.bias[c], 0.f);
-                        else v = __bfloat162float(mv[k]) > 0.f ? v : 0.f;
-                        o[k] = __float2bfloat16_rn(v);
+                    for (int c = 0; c < COUT; ++c)
+                        if (c < a.cout_real) y[c] = __uint_as_float(r[q][c]) + a.bias[c];   // the caller's buffer: float-aligned
+                } else {
+                    uint4* y = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + p * COUT);
+                    const uint4* mk = EPI == kDgrad ? reinterpret_cast<const uint4*>(a.mask + p * COUT) : nullptr;
+#pragma unroll
+                    for (int c8 = 0; c8 < COUT / 8; ++c8) {
+                        __align__(16) bf16 o[8];
+                        __align__(16) bf16 mv[8];
+                        if (EPI == kDgrad) *reinterpret_cast<uint4*>(mv) = mk[c8];
+#pragma unroll
+                        for (int e = 0; e < 8; ++e) {
+                            const int c = 8 * c8 + e;
+                            float v = __uint_as_float(r[q][c]);
+                            if (EPI == kHidden) v = fmaxf(v + a.bias[c], 0.f);
+                            else v = __bfloat162float(mv[e]) > 0.f ? v : 0.f;
+                            o[e] = __float2bfloat16_rn(v);
+                        }
+                        y[c8] = *reinterpret_cast<const uint4*>(o);
                     }
-                    y[c8] = *reinterpret_cast<const uint4*>(o);
                 }
             }
         }
-        tc_fence_before();
-        __syncthreads();   // accumulator read and patch consumed before the next tile
     }
+    if (!ok) atomicExch(a.err, 1);
+    __syncwarp();
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     __syncwarp();
-    if (warp == 0) tmem_dealloc(tmem, 32);
+    if (warp == 0) tmem_dealloc(tmem, G::tmem_cols);
 }
 
 template <int CIN, int COUT, int EPI>
@@ -304,12 +396,11 @@ cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
     // the shared-memory opt-in is a per-device setting: set on the current
     // device at every launch (a host-side call; a few launches per step);
     // if it is refused nothing is launched and the caller reports it
-    const cudaError_t e = cudaFuncSetAttribute(k_conv5<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                               bytes);
+    const cudaError_t e =
+        cudaFuncSetAttribute(k_conv5<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    const int tiles = a.n * a.H * ((a.W + kTile - 1) / kTile);
-    const int grid = tiles < 2 * sms ? tiles : 2 * sms;
-    k_conv5<CIN, COUT, EPI><<<grid, kThreadsConv, bytes, s>>>(a);
+    const int count = Items(a.n, a.H, a.W).count;
+    k_conv5<CIN, COUT, EPI><<<count < sms ? count : sms, kThreadsConv, bytes, s>>>(a);
     return cudaSuccess;
 }
 
@@ -319,30 +410,40 @@ cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
 // s(dx, dz) = (dx - 2, dz - 2).  The pixels are the GEMM's K dimension, so
 // the operand that carries the tap shift must move along K by whole 16-byte
 // rows: both operands use the no-swizzle MN-major layout, in which K
-// advances 16 bytes per pixel.  Per 128-pixel tile (one image row, as in
-// k_conv5) the CTA stages
-//   * the input patch, rows h-2..h+2 (plus zero rows up to 8) and columns
-//     z0-2..z0+129, as [row][channel chunk of 8][column][8 channels] -- the
-//     layout of k_conv5 -- so that M = 128 consecutive 8-channel groups are
-//     (row, chunk) pairs at one uniform stride: 4 rows x 32 channels (or 8 x
-//     16), and the tap shift dz is a start offset of 16 dz bytes;
-//   * the output gradient of the tile, [chunk of 8 output channels][pixel]
-//     [8 channels], the N operand;
-// and one thread issues, for each dz and row group, 8 MMAs of K = 16
-// (kind::f16, BF16 inputs, FP32 accumulation in tensor memory): D[(dx, ci)]
-// [co] for the tile's pixels, accumulated over all of the CTA's tiles.  At
-// the end each warp reads its 32 accumulator lanes (rows (dx, ci)) and
-// writes the CTA's partial sums, which k_wgrad_sum adds in CTA order: the
-// result does not depend on scheduling, so training repeats bit for bit.
+// advances 16 bytes per pixel.  Per work item (kRB rows of 128 pixels) the
+// copy warps bring
+//   * the input patch, rows h-2..h+kRB+1 and columns z0-2..z0+129, as [row]
+//     [channel chunk of 8][column][8 channels] -- the layout of k_conv5 -- so
+//     that M = 128 consecutive 8-channel groups are (row, chunk) pairs at one
+//     uniform stride: 4 rows x 32 channels (or 8 x 16), and the tap shift dz
+//     is a start offset of 16 dz bytes.  The last row group of a pixel row
+//     reads up to three rows beyond the five taps (whatever the buffer holds
+//     there); their accumulator rows are never read;
+//   * the output gradient of the tile, [row][chunk of 8 output channels]
+//     [pixel][8 channels] with zeros beyond the row's end, the N operand;
+// and one thread issues, for each row, 16 pixels, dz and row group, an MMA
+// (kind::f16, BF16 inputs, FP32 accumulation in tensor memory):
+// D[(dx, ci)][co], accumulated over all of the CTA's items.  Copies and MMAs
+// of consecutive items overlap (two stages).  At the end each warp reads its
+// 32 accumulator lanes (rows (dx, ci)) and writes the CTA's partial sums,
+// which k_grad_sum adds in CTA order: the result does not depend on
+// scheduling, so training repeats bit for bit.
+//
+// Bound: the MMAs, as above (3 of 8 rows are spent on the padding above).
+// 32 -> 32, 4 images of 290 x 158: 370 -> 50 us
+// (first form: 64 CTAs that staged and multiplied in turn).
 template <int CIN, int COUT>
 struct WgradGeo {
     static constexpr int NQ = CIN / 8;                  // input-channel chunks
     static constexpr int RPG = 128 / CIN;               // patch rows per M = 128 row group
     static constexpr int NRG = (5 + RPG - 1) / RPG;     // row groups covering dx = 0..4
-    static constexpr int PR = NRG * RPG;                // patch rows held (rows >= 5 stay zero)
-    static constexpr int p_bytes = PR * NQ * kPC * 16;
-    static constexpr int g_bytes = (COUT / 8) * kTile * 16;
-    static constexpr int bytes = p_bytes + g_bytes;
+    static constexpr int row_bytes = NQ * kPC * 16;
+    static constexpr int p_bytes = (kRB + 4) * row_bytes;          // one stage
+    static constexpr int slack = (NRG * RPG - 5) * row_bytes;      // rows read beyond the last stage's patch
+    static constexpr int g_bytes = kRB * (COUT / 8) * kTile * 16;  // one stage
+    static constexpr int oG = 2 * p_bytes + slack;
+    static constexpr int bytes = oG + 2 * g_bytes;
+    static_assert(row_bytes % 128 == 0 && oG % 128 == 0, "tensor-copy destinations are 128-byte aligned");
     static constexpr int ncols = 5 * NRG * COUT;        // accumulator columns
     static constexpr int tmem_cols = ncols <= 32 ? 32 : ncols <= 64 ? 64 : ncols <= 128 ? 128 : ncols <= 256 ? 256 : 512;
     static_assert(ncols <= 512, "accumulators fit tensor memory");
@@ -361,86 +462,84 @@ __device__ __forceinline__ uint64_t umma_desc_mn(uint32_t saddr, uint32_t kgroup
 }
 
 template <int CIN, int COUT>
-__global__ void __launch_bounds__(kThreadsConv) k_wgrad_tc(int n, int H, int W, const bf16* x, const bf16* g,
-                                                        int cin_real, int cout_real, float* part, int* err) {
+__global__ void __launch_bounds__(kThreadsConv, 1) k_wgrad_tc(int n, int H, int W, const bf16* x, const bf16* g,
+                                                           int cin_real, int cout_real, float* part, int* err) {
     using G = WgradGeo<CIN, COUT>;
-    constexpr int NQ = G::NQ, NRG = G::NRG, PR = G::PR, QO = COUT / 8;
+    constexpr int NQ = G::NQ, NRG = G::NRG, QO = COUT / 8;
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* s_p = smem;
-    uint8_t* s_g = smem + G::p_bytes;
-    __shared__ __align__(8) uint64_t bar;
+    uint8_t* s_g = smem + G::oG;
+    __shared__ __align__(8) uint64_t full[2], done[2];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const Items items(n, H, W);
+    const int mine = items.count > (int)blockIdx.x ? (items.count - 1 - blockIdx.x) / gridDim.x + 1 : 0;   // items of this CTA
 
-    // patch rows 5 .. PR-1 are read by the last row group's MMAs and stay zero
-    for (int i = tid; i < (PR - 5) * NQ * kPC; i += kThreadsConv)
-        reinterpret_cast<uint4*>(s_p + 5 * NQ * kPC * 16)[i] = make_uint4(0u, 0u, 0u, 0u);
-    if (tid == 0) mbar_init(&bar, 1);
+    if (tid == 0)
+        for (int s = 0; s < 2; ++s) {
+            mbar_init(&full[s], kCopyThreads);
+            mbar_init(&done[s], 1);
+        }
     __syncwarp();
     if (warp == 0) tmem_alloc(&tmem_base, G::tmem_cols);
     tc_fence_before();
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem = tmem_base;
-    const int tiles_w = (W + kTile - 1) / kTile;
-    const int ntiles = n * H * tiles_w;
-    uint32_t phase = 0, acc = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
-        const int tw = tile % tiles_w, row = tile / tiles_w;
-        const int img = row / H, h = row - img * H;
-        const int z0 = tw * kTile;
-        for (int i = tid; i < 5 * kPC * NQ; i += kThreadsConv) {
-            const int q = i % NQ, rest = i / NQ, c = rest % kPC, r = rest / kPC;
-            const int gh = h + r - 2, gz = z0 + c - 2;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);
-            if (gh >= 0 && gh < H && gz >= 0 && gz < W)
-                v = *reinterpret_cast<const uint4*>(x + (((size_t)img * H + gh) * W + gz) * CIN + q * 8);
-            *reinterpret_cast<uint4*>(s_p + ((size_t)(r * NQ + q) * kPC + c) * 16) = v;
+    if (warp >= 5) {   // copies, as in k_conv5
+        int k = 0;
+        for (; k < mine; ++k) {
+            const int s = k & 1;
+            if (k > 0) hand_over(&full[s ^ 1]);
+            if (k >= 2 && !(ok = mbar_wait(&done[s], (uint32_t)((k >> 1) - 1) & 1u))) break;
+            int img, h, z0;
+            items.at(blockIdx.x + k * gridDim.x, img, h, z0);
+            copy_patch<CIN, kRB + 4, kPC>(smem_u32(s_p) + s * G::p_bytes, x, img, h - 2, z0 - 2, H, W, tid - 160);
+            copy_patch<COUT, kRB, kTile>(smem_u32(s_g) + s * G::g_bytes, g, img, h, z0, H, W, tid - 160);
+            cp_commit();
         }
-        for (int i = tid; i < kTile * QO; i += kThreadsConv) {
-            const int q = i % QO, c = i / QO, gz = z0 + c;
-            uint4 v = make_uint4(0u, 0u, 0u, 0u);   // pixels beyond the row add nothing
-            if (gz < W) v = *reinterpret_cast<const uint4*>(g + (((size_t)img * H + h) * W + gz) * COUT + q * 8);
-            *reinterpret_cast<uint4*>(s_g + ((size_t)q * kTile + c) * 16) = v;
-        }
-        fence_proxy_async();
-        tc_fence_before();
-        __syncthreads();
-        tc_fence_after();
-        if (tid == 0) {
-            const uint32_t pb = smem_u32(s_p), gb = smem_u32(s_g);
-            constexpr uint32_t idesc = idesc_bf16_mn(128, COUT);
+        if (k > 0 && ok) hand_over(&full[(k - 1) & 1]);
+    } else if (tid == 128) {   // MMAs
+        constexpr uint32_t idesc = idesc_bf16_mn(128, COUT);
+        uint32_t acc = 0;
+        for (int k = 0; k < mine; ++k) {
+            const int s = k & 1;
+            ok = mbar_wait(&full[s], (uint32_t)(k >> 1) & 1u);
+            if (!ok) break;
+            tc_fence_after();
+            int img, h, z0;
+            items.at(blockIdx.x + k * gridDim.x, img, h, z0);
+            const int ksn = min(kTile, W - z0 + 15) / 16;   // 16-pixel steps that hold pixels of the row
+            const uint64_t ad0 = umma_desc_mn(smem_u32(s_p) + s * G::p_bytes, 128, kPC * 16);
+            const uint64_t bd0 = umma_desc_mn(smem_u32(s_g) + s * G::g_bytes, 128, kTile * 16);
 #pragma unroll 1
-            for (int dz = 0; dz < 5; ++dz) {
+            for (int r = 0; r < kRB && h + r < H; ++r) {
+                const uint64_t adr = ad0 + (uint32_t)(r * NQ * kPC), bdr = bd0 + (uint32_t)(r * QO * kTile);
+                // consecutive MMAs go to different accumulators
 #pragma unroll 1
-                for (int rg = 0; rg < NRG; ++rg) {
-                    const uint32_t d = tmem + (uint32_t)((dz * NRG + rg) * COUT);
+                for (int ks = 0; ks < ksn; ++ks) {
 #pragma unroll
-                    for (int ks = 0; ks < kTile / 16; ++ks) {
-                        const uint64_t ad = umma_desc_mn(pb + ((rg * G::RPG * NQ) * kPC + dz + 16 * ks) * 16, 128,
-                                                         kPC * 16);
-                        const uint64_t bd = umma_desc_mn(gb + (16 * ks) * 16, 128, kTile * 16);
-                        umma_bf16(d, ad, bd, idesc, (acc | (uint32_t)ks) ? 1u : 0u);
+                    for (int dz = 0; dz < 5; ++dz) {
+#pragma unroll
+                        for (int rg = 0; rg < NRG; ++rg)
+                            umma_bf16(tmem + (uint32_t)((dz * NRG + rg) * COUT), adr + (uint32_t)(rg * G::RPG * NQ * kPC + dz + 16 * ks),
+                                      bdr + (uint32_t)(16 * ks), idesc, acc);
                     }
+                    acc = 1;
                 }
             }
-            umma_commit(&bar);
+            umma_commit(&done[s]);
         }
-        acc = 1;
-        const bool done = mbar_wait(&bar, phase);
-        phase ^= 1u;
-        if (!__syncthreads_and(done)) {
-            if (tid == 0) atomicExch(err, 1);
-            mbar_wait(&bar, phase ^ 1u);   // one more bounded wait for the MMAs in flight
-            ok = false;
-            break;
-        }
+        for (int q = mine - 2 > 0 ? mine - 2 : 0; q < mine && ok; ++q) ok = mbar_wait(&done[q & 1], (uint32_t)(q >> 1) & 1u);
     }
+    if (!ok) atomicExch(err, 1);
+    tc_fence_before();
+    ok = __syncthreads_and(ok);
     tc_fence_after();
     // accumulator row m = 32 warp + lane: 8-channel group j = m / 8 = (row in
     // group, chunk), channel e = m % 8; column (dz, rg) * COUT + co
-    if (ok) {
+    if (ok && mine > 0 && warp < 4) {
         const int m = warp * 32 + lane, j = m >> 3, e = m & 7;
         const int ci = (j % NQ) * 8 + e;
 #pragma unroll 1
@@ -474,9 +573,8 @@ cudaError_t launch_wgrad(int n, int H, int W, const bf16* x, const bf16* g, int 
     constexpr int bytes = WgradGeo<CIN, COUT>::bytes;
     const cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    const int tiles = n * H * ((W + kTile - 1) / kTile);
-    // a fixed grid (at most kMaxRowBlocks partial-sum slots), independent of the device
-    const int grid = tiles < kMaxRowBlocks ? tiles : kMaxRowBlocks;
+    // a fixed grid (at most kWgradCtas partial-sum slots), independent of the device
+    const int count = Items(n, H, W).count, grid = count < kWgradCtas ? count : kWgradCtas;
     k_wgrad_tc<CIN, COUT><<<grid, kThreadsConv, bytes, s>>>(n, H, W, x, g, cin_real, cout_real, part, err);
     *nblocks = grid;
     return cudaSuccess;
@@ -484,50 +582,87 @@ cudaError_t launch_wgrad(int n, int H, int W, const bf16* x, const bf16* g, int 
 
 // ---- gradient sums, bias gradients, packing, Adam ---------------------------
 
-// dw[co][ci][tap] += sum over the CTAs' partial sums, in CTA order.
-__global__ void k_wgrad_sum(int nblocks, int cin_real, int cout_real, const float* part, float* dw) {
-    const int npairs = cin_real * cout_real;
-    for (int i = threadIdx.x + blockIdx.x * blockDim.x; i < kTaps * npairs; i += blockDim.x * gridDim.x) {
-        const int tap = i / npairs, pr = i - tap * npairs;
-        float s = 0.f;
-        for (int b = 0; b < nblocks; ++b) s += part[((size_t)b * kTaps + tap) * kMaxPairs + pr];
-        const int ci = pr % cin_real, co = pr / cin_real;
-        dw[((size_t)co * cin_real + ci) * kTaps + tap] += s;
-    }
-}
-
+// Per-block sums of the output gradient's channels: a thread adds one chunk
+// of 8 channels over its pixels, then the block adds its threads in a fixed
+// order.  part[block][32].
 template <int COUT>
-__global__ void k_bgrad(size_t npix, const bf16* g, int cout_real, float* part) {
-    float acc[COUT];
+__global__ void __launch_bounds__(256) k_bgrad(size_t npix, const bf16* g, float* part) {
+    constexpr int QO = COUT / 8;
+    float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+    const uint4* g4 = reinterpret_cast<const uint4*>(g);
+    const size_t n4 = npix * QO;   // the stride is a multiple of QO: a thread keeps its chunk
+    for (size_t i = threadIdx.x + (size_t)blockIdx.x * 256; i < n4; i += (size_t)256 * gridDim.x) {
+        const uint4 u = g4[i];
+        __align__(16) bf16 v[8];
+        *reinterpret_cast<uint4*>(v) = u;
 #pragma unroll
-    for (int c = 0; c < COUT; ++c) acc[c] = 0.f;
-    for (size_t p = threadIdx.x + (size_t)blockIdx.x * blockDim.x; p < npix; p += (size_t)blockDim.x * gridDim.x)
+        for (int e = 0; e < 8; ++e) acc[e] += __bfloat162float(v[e]);
+    }
+    __shared__ float red[8][32];
+    const int w = threadIdx.x >> 5, lane = threadIdx.x & 31;
 #pragma unroll
-        for (int c = 0; c < COUT; ++c) acc[c] += __bfloat162float(g[p * COUT + c]);
-    const int wid = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5);
-    for (int c = 0; c < cout_real; ++c) {
-        float v = acc[c];
+    for (int e = 0; e < 8; ++e) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-        if ((threadIdx.x & 31) == 0) part[(size_t)wid * 32 + c] = v;   // one slot per warp and channel
+        for (int o = 16; o >= QO; o >>= 1) acc[e] += __shfl_xor_sync(0xffffffffu, acc[e], o);
+        if (lane < QO) red[w][lane * 8 + e] = acc[e];
+    }
+    __syncthreads();
+    if (threadIdx.x < COUT) {
+        float s = 0.f;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) s += red[k][threadIdx.x];
+        part[(size_t)blockIdx.x * 32 + threadIdx.x] = s;
     }
 }
 
-// db[c] += sum over the warps' partial sums, in warp order.
-__global__ void k_bgrad_sum(int nwarps, int cout_real, const float* part, float* db) {
-    const int c = threadIdx.x;
-    if (c >= cout_real) return;
+// dw[co][ci][tap] += the CTAs' partial sums in a fixed order: four threads
+// each add a quarter of the CTAs in order, then the four; the last block
+// adds the bias sums, a warp per channel, lanes striding the blocks and a
+// fixed tree over the lanes.
+__global__ void __launch_bounds__(256) k_grad_sum(int nblocks, int cin_real, int cout_real, const float* part, float* dw,
+                                                  int nbias, const float* bpart, float* db) {
+    if (blockIdx.x == gridDim.x - 1) {
+        const int lane = threadIdx.x & 31;
+        for (int c = threadIdx.x >> 5; c < cout_real; c += 8) {
+            float s = 0.f;
+#pragma unroll 4
+            for (int b = lane; b < nbias; b += 32) s += bpart[(size_t)b * 32 + c];
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+            if (lane == 0) db[c] += s;
+        }
+        return;
+    }
+    __shared__ float red[4][64];
+    const int npairs = cin_real * cout_real, grp = threadIdx.x >> 6, t = threadIdx.x & 63;
+    const int i = blockIdx.x * 64 + t;
+    const bool in = i < kTaps * npairs;
+    const int tap = in ? i / npairs : 0, pr = in ? i - tap * npairs : 0;
+    const float* p = part + (size_t)tap * kMaxPairs + pr;
+    const int b0 = nblocks * grp / 4, b1 = nblocks * (grp + 1) / 4;
     float s = 0.f;
-    for (int w = 0; w < nwarps; ++w) s += part[(size_t)w * 32 + c];
-    db[c] += s;
+#pragma unroll 8
+    for (int b = b0; b < b1; ++b) s += p[(size_t)b * kTaps * kMaxPairs];
+    red[grp][t] = s;
+    __syncthreads();
+    if (grp == 0 && in) {
+        const int ci = pr % cin_real, co = pr / cin_real;
+        dw[((size_t)co * cin_real + ci) * kTaps + tap] += ((red[0][t] + red[1][t]) + red[2][t]) + red[3][t];
+    }
 }
 
-// float [P][creal] -> bf16 [P][cpad], zero-padded channels
-__global__ void k_to_bf16(size_t npix, int creal, int cpad, const float* in, bf16* out) {
-    for (size_t i = threadIdx.x + (size_t)blockIdx.x * blockDim.x; i < npix * cpad; i += (size_t)blockDim.x * gridDim.x) {
-        const size_t p = i / cpad;
-        const int c = (int)(i % cpad);
-        out[i] = __float2bfloat16_rn(c < creal ? in[p * creal + c] : 0.f);
+// float [P][CREAL] -> bf16 [P][16], zero-padded channels; a thread per pixel.
+template <int CREAL>
+__global__ void __launch_bounds__(256) k_to_bf16(size_t npix, const float* in, bf16* out) {
+    static_assert(CREAL <= 16, "padded to 16 channels");
+    for (size_t p = threadIdx.x + (size_t)blockIdx.x * 256; p < npix; p += (size_t)256 * gridDim.x) {
+        __align__(16) bf16 o[16];
+        const float* f = in + p * CREAL;
+#pragma unroll
+        for (int c = 0; c < 16; ++c) o[c] = __float2bfloat16_rn(c < CREAL ? f[c] : 0.f);   // only float alignment is known
+        uint4* y = reinterpret_cast<uint4*>(out + p * 16);
+        y[0] = reinterpret_cast<const uint4*>(o)[0];
+        y[1] = reinterpret_cast<const uint4*>(o)[1];
     }
 }
 
@@ -599,7 +734,8 @@ struct ouc_cnn {
     bf16* wf[4] = {};            // packed forward weights
     bf16* wd[4] = {};            // packed input-gradient weights (layers 1..3)
     int* err = nullptr;
-    float* part = nullptr;       // gradient partial sums, reduced in a fixed order (kMaxRowBlocks x 25 x kMaxPairs)
+    float* part = nullptr;       // gradient partial sums, reduced in a fixed order (kWgradCtas x 25 x kMaxPairs)
+    float* bpart = nullptr;      // bias partial sums (kBgradBlocks x 32)
     // activations of the last forward
     int n = 0, H = 0, W = 0;
     size_t cap = 0;              // pixels the buffers hold
@@ -664,7 +800,8 @@ int ouc_cnn_create(int device, ouc_cnn** out) {
     bool ok = cudaMalloc(&net->params, pb) == cudaSuccess && cudaMalloc(&net->grads, pb) == cudaSuccess &&
               cudaMalloc(&net->adam_m, pb) == cudaSuccess && cudaMalloc(&net->adam_v, pb) == cudaSuccess &&
               cudaMalloc(&net->err, sizeof(int)) == cudaSuccess &&
-              cudaMalloc(&net->part, (size_t)kMaxRowBlocks * kTaps * kMaxPairs * sizeof(float)) == cudaSuccess;
+              cudaMalloc(&net->part, (size_t)kWgradCtas * kTaps * kMaxPairs * sizeof(float)) == cudaSuccess &&
+              cudaMalloc(&net->bpart, (size_t)kBgradBlocks * 32 * sizeof(float)) == cudaSuccess;
     for (int l = 0; l < 4 && ok; ++l) {
         ok = cudaMalloc(&net->wf[l], (size_t)kTaps * kL[l].cin_pad * kL[l].cout_pad * 2) == cudaSuccess;
         if (ok && l > 0) ok = cudaMalloc(&net->wd[l], (size_t)kTaps * kL[l].cin_pad * kL[l].cout_pad * 2) == cudaSuccess;
@@ -691,7 +828,7 @@ int ouc_cnn_destroy(ouc_cnn* net) {
     if (!net) return OUC_OK;
     cudaSetDevice(net->device);
     cudaDeviceSynchronize();
-    cudaFree(net->params); cudaFree(net->grads); cudaFree(net->adam_m); cudaFree(net->adam_v); cudaFree(net->err); cudaFree(net->part);
+    cudaFree(net->params); cudaFree(net->grads); cudaFree(net->adam_m); cudaFree(net->adam_v); cudaFree(net->err); cudaFree(net->part); cudaFree(net->bpart);
     for (auto* p : net->wf) cudaFree(p);
     for (auto* p : net->wd) cudaFree(p);
     cudaFree(net->x0); cudaFree(net->g16);
@@ -723,7 +860,7 @@ int ouc_cnn_forward_dev(ouc_cnn* net, int n, int H, int W, const float* d_in, fl
     const size_t P = (size_t)n * H * W;
     if (ensure_acts(net, P)) return OUC_ENOMEM;
     net->n = n; net->H = H; net->W = W;
-    k_to_bf16<<<1024, 256, 0, s>>>(P, OUC_CNN_IN, 16, d_in, net->x0);
+    k_to_bf16<OUC_CNN_IN><<<1184, 256, 0, s>>>(P, d_in, net->x0);
     ConvArgs a{};
     a.n = n; a.H = H; a.W = W; a.err = net->err;
     a.x = net->x0; a.w = net->wf[0]; a.bias = net->params + p_offset(0) + w_count(0); a.y = net->y[0];
@@ -746,15 +883,15 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
     const int n = net->n, H = net->H, W = net->W;
     const size_t P = (size_t)n * H * W;
     int nb = 0;   // CTAs of the weight-gradient launch: partial-sum slots to add
-    k_to_bf16<<<1024, 256, 0, s>>>(P, OUC_CNN_OUT, 16, d_gout, net->g16);
+    k_to_bf16<OUC_CNN_OUT><<<1184, 256, 0, s>>>(P, d_gout, net->g16);
     // layer 4: weights and bias, then the gradient into layer 3's output
     float* gp = net->grads;
     if (launch_wgrad<32, 16>(n, H, W, net->y[2], net->g16, kL[3].cin, kL[3].cout, net->part, net->err, &nb, s) !=
         cudaSuccess)
         return OUC_ECUDA;
-    k_wgrad_sum<<<64, 256, 0, s>>>(nb, kL[3].cin, kL[3].cout, net->part, gp + p_offset(3));
-    k_bgrad<16><<<kBgradBlocks, 256, 0, s>>>(P, net->g16, kL[3].cout, net->part);
-    k_bgrad_sum<<<1, 32, 0, s>>>(kBgradBlocks * 8, kL[3].cout, net->part, gp + p_offset(3) + w_count(3));
+    k_bgrad<16><<<kBgradBlocks, 256, 0, s>>>(P, net->g16, net->bpart);
+    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[3].cin, kL[3].cout, net->part, gp + p_offset(3), kBgradBlocks, net->bpart,
+                                   gp + p_offset(3) + w_count(3));
     ConvArgs a{};
     a.n = n; a.H = H; a.W = W; a.err = net->err;
     a.x = net->g16; a.w = net->wd[3]; a.mask = net->y[2]; a.y = net->g[0];
@@ -765,9 +902,9 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
         if (launch_wgrad<32, 32>(n, H, W, net->y[l - 1], gl, kL[l].cin, kL[l].cout, net->part, net->err, &nb, s) !=
             cudaSuccess)
             return OUC_ECUDA;
-        k_wgrad_sum<<<64, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l));
-        k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, gl, kL[l].cout, net->part);
-        k_bgrad_sum<<<1, 32, 0, s>>>(kBgradBlocks * 8, kL[l].cout, net->part, gp + p_offset(l) + w_count(l));
+        k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, gl, net->bpart);
+    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l), kBgradBlocks, net->bpart,
+                                   gp + p_offset(l) + w_count(l));
         a.x = gl; a.w = net->wd[l]; a.mask = net->y[l - 1]; a.y = net->g[(3 - l) & 1];
         if (launch_conv<32, 32, kDgrad>(a, net->sms, s) != cudaSuccess) return OUC_ECUDA;
     }
@@ -775,9 +912,9 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
     const bf16* g1 = net->g[0];
     if (launch_wgrad<16, 32>(n, H, W, net->x0, g1, kL[0].cin, kL[0].cout, net->part, net->err, &nb, s) != cudaSuccess)
         return OUC_ECUDA;
-    k_wgrad_sum<<<64, 256, 0, s>>>(nb, kL[0].cin, kL[0].cout, net->part, gp + p_offset(0));
-    k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, g1, kL[0].cout, net->part);
-    k_bgrad_sum<<<1, 32, 0, s>>>(kBgradBlocks * 8, kL[0].cout, net->part, gp + p_offset(0) + w_count(0));
+    k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, g1, net->bpart);
+    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[0].cin, kL[0].cout, net->part, gp + p_offset(0), kBgradBlocks, net->bpart,
+                                   gp + p_offset(0) + w_count(0));
     return cudaGetLastError() == cudaSuccess ? OUC_OK : OUC_ECUDA;
 }
 

@@ -234,26 +234,23 @@ int launch_back(int N, const StepArgs& rec, const StepArgs& rcv, int nshots, cud
     return 1;
 }
 
-namespace {
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
-                                 const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
-                                 CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-EncodeTiled encoder() {
-    static EncodeTiled fn = []() -> EncodeTiled {
+TensorMapEncode tensor_map_encoder() {
+    static TensorMapEncode fn = []() -> TensorMapEncode {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
         if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
             q != cudaDriverEntryPointSuccess)
             return nullptr;
-        return reinterpret_cast<EncodeTiled>(p);
+        return reinterpret_cast<TensorMapEncode>(p);
     }();
     return fn;
 }
 
+namespace {
 template <int N>
 cudaError_t encode_for(StepArgs& a, const float* state0, int pitch, int rows, int nfields, int nslots, size_t fstride) {
     using G = TileGeo<N>;
-    EncodeTiled enc = encoder();
+    TensorMapEncode enc = tensor_map_encoder();
     if (!enc) return cudaErrorNotSupported;
     // dimensions innermost first: columns, rows, fields, slots; strides in bytes
     const cuuint64_t dims[4] = {(cuuint64_t)pitch, (cuuint64_t)rows, (cuuint64_t)nfields, (cuuint64_t)nslots};

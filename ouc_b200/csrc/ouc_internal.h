@@ -275,6 +275,12 @@ struct GradStackArgs {
     double* stack[3];        // nx*nz dense FP64
 };
 
+// cuTensorMapEncodeTiled, reached through the runtime (null if the driver lacks it).
+using TensorMapEncode = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
+                                     const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
+                                     CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+TensorMapEncode tensor_map_encoder();
+
 // Host-side launchers (kernels.cu)
 // Encode StepArgs::box_map for a state block at `state0` (nslots shot slots
 // of nfields fields of rows x pitch floats each) and half-order N.
