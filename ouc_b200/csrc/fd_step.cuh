@@ -307,6 +307,22 @@ __device__ __forceinline__ void tma_prefetch_box4(const CUtensorMap* map, int c0
 // launch was an ordinary one).
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// Launch with programmatic stream serialization: the kernel may start before
+// the launch ahead of it in the stream has finished (pdl_wait orders them).
+template <class... P, class... A>
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, const A&... args) {
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t c = {};
+    c.gridDim = grid;
+    c.blockDim = dim3(threads);
+    c.dynamicSmemBytes = smem;
+    c.stream = s;
+    c.attrs = at;
+    c.numAttrs = 1;
+    cudaLaunchKernelEx(&c, kernel, args...);
+}
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
 
 // Per-launch, per-shot constants.
@@ -634,21 +650,25 @@ __device__ __forceinline__ const CUtensorMap* u_map(const StepArgs& p) {
 // launch, which is its slot in the state block (its fields lie slot x
 // shot_stride floats after shot 0's).
 template <class G>
-__device__ __forceinline__ void issue_u_box(const StepArgs& p, float* sm, int x0, int z0, int slot, uint64_t* bar) {
-    const CUtensorMap* map = u_map<G>(p);
+__device__ __forceinline__ void issue_box(const CUtensorMap* map, const int (&field)[4], unsigned tx_extra, float* sm, int x0,
+                                          int z0, int slot, uint64_t* bar) {
     static_assert(G::floats - G::oTh >= 2 * G::UR * G::UC, "S staging fits the S-stage area");
     static_assert((G::oUz * 4) % 128 == 0 && (G::oTh * 4) % 128 == 0 && (G::UR * G::UC * 4) % 128 == 0,
                   "tensor-copy destinations are 128-byte aligned");
-    mbar_arrive_tx(bar, 4u * G::UR * G::UC * 4u + p.copy_tx_extra);
+    mbar_arrive_tx(bar, 4u * G::UR * G::UC * 4u + tx_extra);
     // a previous tile's shared-memory accesses (generic proxy) precede these writes
     fence_proxy_async();
     // allocation coordinates: column z0 - HU + kZOFF (a multiple of 4), row x0 - SHX - N + kGX (>= 0)
     const int c0 = z0 - G::HU + kZOFF, c1 = x0 - G::SHX - G::N + kGX;
     float* stS = sm + G::oTh;
-    tma_box4(sm + G::oUx, map, c0, c1, p.now_field[0], slot, bar);
-    tma_box4(sm + G::oUz, map, c0, c1, p.now_field[1], slot, bar);
-    tma_box4(stS, map, c0, c1, p.now_field[2], slot, bar);
-    tma_box4(stS + G::UR * G::UC, map, c0, c1, p.now_field[3], slot, bar);
+    tma_box4(sm + G::oUx, map, c0, c1, field[0], slot, bar);
+    tma_box4(sm + G::oUz, map, c0, c1, field[1], slot, bar);
+    tma_box4(stS, map, c0, c1, field[2], slot, bar);
+    tma_box4(stS + G::UR * G::UC, map, c0, c1, field[3], slot, bar);
+}
+template <class G>
+__device__ __forceinline__ void issue_u_box(const StepArgs& p, float* sm, int x0, int z0, int slot, uint64_t* bar) {
+    issue_box<G>(u_map<G>(p), p.now_field, p.copy_tx_extra, sm, x0, z0, slot, bar);
 }
 
 // Offsets within one field are 32-bit ints (row * pitch + column, guard rows

@@ -5,7 +5,8 @@
 // State: the P/S velocity parts (Vpx, Vpz, Vsx, Vsz) and eight split stresses
 // (theta_x, theta_z, omega_x, omega_z and the four Q fields), each
 // ping-ponged so that the halo reads of one step never meet its writes.  One
-// 32 x 64 tile per CTA, in three phases like the second-order step kernel:
+// tile per CTA (32 x 64, 16 x 64 or the small tiles of fd_small.cuh, chosen
+// as for the second-order step), in three phases like that kernel:
 //   1. U = P + S velocity over the tile and a 2N halo into shared memory;
 //   2. the stress update over the tile and an N halo (four staggered velocity
 //      derivatives, the split-field damping (1 - dt a/2)/(1 + dt a/2), the
@@ -24,12 +25,16 @@
 
 #include "../../include/ouc.h"
 #include "ctx.h"
+#include "fd_small.cuh"
 #include "fd_step.cuh"
 
 namespace ouc {
 namespace fo {
 
 struct FoArgs {
+    alignas(64) CUtensorMap map;     // U box of the launch's tile over the state block
+    int vfield[4];                   // fields of vold[] in the block
+    int* err;                        // device status word (bit 0: a copy wait ran out)
     int X, Z, pitch, tiles_z, t, nt;
     int sx, sz, rz;                  // padded source cell and receiver row
     float a[6];
@@ -77,11 +82,89 @@ __global__ void k_squares(const float* __restrict__ vp, const float* __restrict_
     }
 }
 
-template <int N>
-__global__ void __launch_bounds__(kThreads, 2) k_fo(const FoArgs p) {
-    using G = TileGeo<N>;
+// Wait for the tile's copies, form U = P + S (and at the receiver row the
+// injected records).  False, with bit 0 of *p.err set, when they did not land.
+template <class G>
+__device__ __forceinline__ bool fo_u_box(const FoArgs& p, float* sm, int x0, int z0, uint64_t* bar) {
+    constexpr int UC = G::UC, NT = G::NT;
+    float* sUx = sm + G::oUx;
+    float* sUz = sm + G::oUz;
+    const float* stS = sm + G::oTh;
+    const int tid = threadIdx.x;
+    const int err_word = *(volatile const int*)p.err;
+    const bool landed = mbar_wait(bar, 0u);
+    if (!__syncthreads_and(landed && !(err_word & 1))) {
+        if (tid == 0) {
+            if (!landed) mbar_wait(bar, 0u);   // copies in flight land before the CTA ends
+            atomicOr(p.err, 1);
+        }
+        __syncthreads();
+        return false;
+    }
+    for (int idx = tid; idx < G::UR * (UC / 4); idx += NT) {
+        st4(sUx + 4 * idx, add4(ld4(sUx + 4 * idx), ld4(stS + 4 * idx)));                // Vx = Vpx + Vsx
+        st4(sUz + 4 * idx, add4(ld4(sUz + 4 * idx), ld4(stS + G::UR * UC + 4 * idx)));
+    }
+    const int ux_i0 = x0 - G::SHX - G::N, col = p.rz - (z0 - G::HU);
+    if (p.inj_x && col >= 0 && col < UC) {
+        // load_record (PS:1472-1481): U at the receiver row replaced by the
+        // records before the stress update reads it
+        __syncthreads();
+        for (int r = tid; r < G::UR; r += NT) {
+            const int gi = ux_i0 + r;
+            if (gi >= p.L && gi < p.X - p.L) {
+                sUx[r * UC + col] = p.inj_x[gi];
+                sUz[r * UC + col] = p.inj_z[gi];
+            }
+        }
+    }
+    __syncthreads();
+    return true;
+}
+
+// Whether the tile's S region meets the x or z damping layers (elsewhere the
+// damping is exactly 0 and its profiles are not read).
+template <class G>
+__device__ __forceinline__ bool fo_damped(const FoArgs& p, int x0, int z0) {
+    return x0 - G::SHX < p.L || x0 + G::TX + G::SHX - 1 >= p.X - p.L || z0 - G::HS < p.L ||
+           z0 + G::TZ + G::HS - 1 >= p.Z - p.L;
+}
+
+// live[k]: cell k of the quad is updated by the reference
+__device__ __forceinline__ unsigned fo_live(const FoArgs& p, int N, int gi, int gj) {
+    unsigned m = 0;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) m |= (gi >= N && gi < p.X - N && gj + k >= N && gj + k < p.Z - N) ? (1u << k) : 0u;
+    return m;
+}
+__device__ __forceinline__ float4 fo_mask(float4 v, unsigned live) {
+    return make_float4(live & 1u ? v.x : 0.f, live & 2u ? v.y : 0.f, live & 4u ? v.z : 0.f, live & 8u ? v.w : 0.f);
+}
+// Products that an addition follows: scalar, since the compiler contracts a
+// packed multiplication with the packed addition after it.
+__device__ __forceinline__ float4 prod4(float4 a, float4 b) {
+    return make_float4(__fmul_rn(a.x, b.x), __fmul_rn(a.y, b.y), __fmul_rn(a.z, b.z), __fmul_rn(a.w, b.w));
+}
+// term + old, or the damped update, of one quad (dd: its damping, 0 where flat)
+__device__ __forceinline__ float4 fo_stress4(bool flat, float4 dd, float dt, float4 term, float4 old) {
+    if (flat) return add4(term, old);
+    return make_float4(stress_upd(dd.x, dt, term.x, old.x), stress_upd(dd.y, dt, term.y, old.y),
+                       stress_upd(dd.z, dt, term.z, old.z), stress_upd(dd.w, dt, term.w, old.w));
+}
+__device__ __forceinline__ float4 fo_vel4(bool flat, float4 dd, float dt, float4 old, float4 sum) {
+    if (flat) return add4(old, prod4(sum, make_float4(dt, dt, dt, dt)));
+    return make_float4(vel_upd(dd.x, dt, old.x, sum.x), vel_upd(dd.y, dt, old.y, sum.y), vel_upd(dd.z, dt, old.z, sum.z),
+                       vel_upd(dd.w, dt, old.w, sum.w));
+}
+__device__ __forceinline__ float4 neg4(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
+
+// Bound: latency and issue, as the second-order step.  1060 x 560, per step:
+// 32 x 64 tiles with plain loads 52 us; 16 x 64 tiles, tensor copies and
+// operands ahead of the derivatives TFO us.
+template <int N, class G>
+__global__ void __launch_bounds__(kThreads, 2) k_fo(const __grid_constant__ FoArgs p) {
     constexpr int TX = G::TX, TZ = G::TZ, SHX = G::SHX, HS = G::HS, HU = G::HU, UC = G::UC, SC = G::SC;
-    extern __shared__ float4 smem4[];
+    extern __shared__ __align__(128) float4 smem4[];
     float* sm = reinterpret_cast<float*>(smem4);
     float* sUx = sm + G::oUx;
     float* sUz = sm + G::oUz;
@@ -91,109 +174,97 @@ __global__ void __launch_bounds__(kThreads, 2) k_fo(const FoArgs p) {
     float* sQzz = sm + G::oQzz;
     float* sQxx = sm + G::oQxx;
     float* sQzx = sm + G::oQzx;
+    __shared__ uint64_t bar;
     const int tid = threadIdx.x;
     const int P = p.pitch;
     const int tz = blockIdx.x % p.tiles_z, tx = blockIdx.x / p.tiles_z;
     const int x0 = tx * TX, z0 = tz * TZ;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_map(&p.map);
+        pdl_wait();
+        issue_box<G>(&p.map, p.vfield, 0u, sm, x0, z0, 0, &bar);
+    }
     float a[N];
 #pragma unroll
     for (int k = 0; k < N; ++k) a[k] = p.a[k];
     const Div dvx = make_div(p.dx, p.rdx), dvz = make_div(p.dz, p.rdz);
     const float dt = p.dt;
-    const int ux_i0 = x0 - SHX - N, ux_j0 = z0 - HU;
+    const bool damped = fo_damped<G>(p, x0, z0);
+    __syncthreads();   // the mbarrier is initialised
+    pdl_wait();
 
     // ---- phase 1: U = P + S velocity over the tile and a 2N halo ----------
-    for (int idx = tid; idx < G::UR * (UC / 4); idx += kThreads) {
-        const int r = idx / (UC / 4), c4 = idx - r * (UC / 4);
-        const int g = (ux_i0 + r) * P + (ux_j0 + 4 * c4);
-        float4 ux = add4(ld4(p.vold[0] + g), ld4(p.vold[2] + g));   // Vx = Vpx + Vsx
-        float4 uz = add4(ld4(p.vold[1] + g), ld4(p.vold[3] + g));
-        const int gi = ux_i0 + r, gj = ux_j0 + 4 * c4;
-        if (p.inj_x && p.rz >= gj && p.rz < gj + 4 && gi >= p.L && gi < p.X - p.L) {
-            // load_record (PS:1472-1481): U at the receiver row replaced by
-            // the records before the stress update reads it
-            set_comp(ux, p.rz - gj, p.inj_x[gi]);
-            set_comp(uz, p.rz - gj, p.inj_z[gi]);
-        }
-        st4(sUx + r * UC + 4 * c4, ux);
-        st4(sUz + r * UC + 4 * c4, uz);
-    }
-    __syncthreads();
+    if (!fo_u_box<G>(p, sm, x0, z0, &bar)) return;
 
     // ---- phase 2: stresses on the tile plus an N halo ----------------------
     if (tid < G::itemsA + G::itemsB) {
         int r0, c;
         const bool groupA = tid < G::itemsA;
         if (groupA) {
-            r0 = -SHX + 4 * (tid / (TZ / 4));
+            r0 = -SHX + G::RS * (tid / (TZ / 4));
             c = 4 * (tid % (TZ / 4));
         } else {
             const int k = tid - G::itemsA;
-            r0 = 4 * (k / (2 * HS / 4));
+            r0 = G::RS * (k / (2 * HS / 4));
             const int cc = k % (2 * HS / 4);
             c = cc < HS / 4 ? -HS + 4 * cc : TZ + 4 * (cc - HS / 4);
         }
         const float* ux0 = sUx + (r0 + SHX + N) * UC + (c + HU);
         const float* uz0 = sUz + (r0 + SHX + N) * UC + (c + HU);
-        float4 exx[4], ezx[4];
-        dx4<N, 4, false>(ux0, UC, a, dvx, exx);   // dvxdx = D-x Vx
-        dx4<N, 4, true>(uz0, UC, a, dvx, ezx);    // dvzdx = D+x Vz
         const bool ownc = c >= 0 && c < TZ;
+#pragma unroll 1
+        for (int q0 = 0; q0 < G::RS; q0 += 2) {
+        float4 exx[2], ezx[2];
+        dx4<N, 2, false>(ux0 + q0 * UC, UC, a, dvx, exx);   // dvxdx = D-x Vx
+        dx4<N, 2, true>(uz0 + q0 * UC, UC, a, dvx, ezx);    // dvzdx = D+x Vz
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = r0 + q, gi = x0 + r, gjb = z0 + c;
+        for (int qq = 0; qq < 2; ++qq) {
+            const int q = q0 + qq, r = r0 + q, gi = x0 + r, gjb = z0 + c;
+            const int g = gi * P + gjb;
+            // operands first: their latency runs under the z derivatives
+            const float4 vp2v = ldg4(p.vp2 + g), vs2v = ldg4(p.vs2 + g);
+            float4 so[8];
+#pragma unroll
+            for (int f = 0; f < 8; ++f) so[f] = ldg4(p.sold[f] + g);
+            float4 axv = zero4(), azv = zero4();
+            if (damped) { axv = ldg4(p.ax + g); azv = ldg4(p.az + g); }
             const float4 exz = dz4<N, true>(ux0 + q * UC, a, dvz);    // dvxdz = D+z Vx
             const float4 ezz = dz4<N, false>(uz0 + q * UC, a, dvz);   // dvzdz = D-z Vz
-            const int g = gi * P + gjb;
-            const float4 vp2v = ld4(p.vp2 + g), vs2v = ld4(p.vs2 + g), axv = ld4(p.ax + g), azv = ld4(p.az + g);
-            float4 so[8], sn[8];
+            const bool flat = !damped || undamped4(axv, azv);
+            // dt Vp^2 d, dt Vs^2 d and -dt Vs^2 d, each rounded as the reference's float products
+            const float4 cp = mul4s(vp2v, dt), cs = mul4s(vs2v, dt), cm = neg4(cs);
+            const unsigned live = fo_live(p, N, gi, gjb);
+            float4 sn[8];
+            sn[0] = fo_stress4(flat, axv, dt, prod4(cp, exx[qq]), so[0]);   // theta_x
+            sn[1] = fo_stress4(flat, azv, dt, prod4(cp, ezz), so[1]);       // theta_z
+            sn[2] = fo_stress4(flat, axv, dt, prod4(cm, ezx[qq]), so[2]);   // omega_x
+            sn[3] = fo_stress4(flat, azv, dt, prod4(cs, exz), so[3]);       // omega_z
+            sn[4] = fo_stress4(flat, axv, dt, prod4(cs, exx[qq]), so[4]);   // Qxx (duxdx)
+            sn[5] = fo_stress4(flat, azv, dt, prod4(cs, exz), so[5]);       // Qxz (duxdz)
+            sn[6] = fo_stress4(flat, axv, dt, prod4(cs, ezx[qq]), so[6]);   // Qzx (duzdx)
+            sn[7] = fo_stress4(flat, azv, dt, prod4(cs, ezz), so[7]);       // Qzz (duzdz)
+            if (live != 0xfu) {
 #pragma unroll
-            for (int f = 0; f < 8; ++f) so[f] = ld4(p.sold[f] + g);
-            const bool row_live = gi >= N && gi < p.X - N;
-            const bool flat = undamped4(axv, azv);
-            float th[4], om[4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int gj = gjb + k;
-                const bool live = row_live && gj >= N && gj < p.Z - N;
-                const float cp = __fmul_rn(dt, comp(vp2v, k)), cs = __fmul_rn(dt, comp(vs2v, k));
-                const float dxx = comp(exx[q], k), dzz = comp(ezz, k), dxz = comp(exz, k), dzx = comp(ezx[q], k);
-                // dt Vp^2 d, dt Vs^2 d and -dt Vs^2 d, each rounded as the reference's float products
-                float term[8];
-                term[0] = __fmul_rn(cp, dxx);    // theta_x
-                term[1] = __fmul_rn(cp, dzz);    // theta_z
-                term[2] = __fmul_rn(-cs, dzx);   // omega_x
-                term[3] = __fmul_rn(cs, dxz);    // omega_z
-                term[4] = __fmul_rn(cs, dxx);    // Qxx (duxdx)
-                term[5] = __fmul_rn(cs, dxz);    // Qxz (duxdz)
-                term[6] = __fmul_rn(cs, dzx);    // Qzx (duzdx)
-                term[7] = __fmul_rn(cs, dzz);    // Qzz (duzdz)
-                float v[8];
-                if (flat) {
-#pragma unroll
-                    for (int f = 0; f < 8; ++f) v[f] = __fadd_rn(term[f], comp(so[f], k));
-                } else {
-                    const float dax = comp(axv, k), daz = comp(azv, k);
-#pragma unroll
-                    for (int f = 0; f < 8; ++f) v[f] = stress_upd((f & 1) ? daz : dax, dt, term[f], comp(so[f], k));
-                }
-#pragma unroll
-                for (int f = 0; f < 8; ++f) {
-                    if (!live) v[f] = 0.f;   // the reference never updates these cells
-                    set_comp(sn[f], k, v[f]);
-                }
-                const float s = (p.wavelet && live && gi == p.sx && gj == p.sz) ? p.wavelet[p.t] : 0.f;
-                th[k] = v[0] + v[1] + s;   // PS:557
-                om[k] = v[2] + v[3];
+                for (int f = 0; f < 8; ++f) sn[f] = fo_mask(sn[f], live);   // the reference never updates these cells
             }
-            const bool own = ownc && r >= 0 && r < TX;
-            if (own) {
+            float4 th = add4(sn[0], sn[1]);
+            const float4 om = add4(sn[2], sn[3]);
+            // theta_x + theta_z + s with s = 0 off the source (PS:557): the
+            // second addition turns -0 into +0
+            float4 sv = zero4();
+            if (p.wavelet && gi == p.sx && p.sz >= gjb && p.sz < gjb + 4 && (live >> (p.sz - gjb) & 1u))
+                set_comp(sv, p.sz - gjb, p.wavelet[p.t]);
+            th = add4(th, sv);
+            if (ownc && r >= 0 && r < TX) {
 #pragma unroll
-                for (int f = 0; f < 8; ++f) st4(p.snew[f] + g, sn[f]);
+                for (int f = 0; f < 8; ++f) stg4(p.snew[f] + g, sn[f]);
             }
             const int sr = r + SHX, scol = c + HS;
-            st4(sTh + sr * SC + scol, make_float4(th[0], th[1], th[2], th[3]));
-            st4(sOm + sr * SC + scol, make_float4(om[0], om[1], om[2], om[3]));
+            st4(sTh + sr * SC + scol, th);
+            st4(sOm + sr * SC + scol, om);
             if (groupA) {
                 st4(sQxz + sr * TZ + c, sn[5]);
                 st4(sQzz + sr * TZ + c, sn[7]);
@@ -203,17 +274,23 @@ __global__ void __launch_bounds__(kThreads, 2) k_fo(const FoArgs p) {
                 st4(sQzx + r * SC + scol, sn[6]);
             }
         }
+        }
     }
     __syncthreads();
 
-    // ---- phase 3: velocities of the own cells (2 rows x 4 columns) ---------
+    // ---- phase 3: velocities of the own cells --------------------------------
     {
-        const int rr = 2 * (tid / (TZ / 4));
+        const int rr = G::RU * (tid / (TZ / 4));
         const int c = 4 * (tid % (TZ / 4));
         const int scol = c + HS;
 #pragma unroll 1
-        for (int q = 0; q < 2; ++q) {
+        for (int q = 0; q < G::RU; ++q) {
             const int r = rr + q, gi = x0 + r;
+            const int g = gi * P + (z0 + c);
+            const float4 opx = ldg4(p.vold[0] + g), opz = ldg4(p.vold[1] + g);
+            const float4 osx = ldg4(p.vold[2] + g), osz = ldg4(p.vold[3] + g);
+            float4 axv = zero4(), azv = zero4();
+            if (damped) { axv = ldg4(p.ax + g); azv = ldg4(p.az + g); }
             float4 txv[1], wxv[1], dB[1], dE[1];
             dx4<N, 1, true>(sTh + (r + SHX) * SC + scol, SC, a, dvx, txv);    // dthetadx = D+x theta
             dx4<N, 1, false>(sOm + (r + SHX) * SC + scol, SC, a, dvx, wxv);   // domegadx = D-x omega
@@ -223,40 +300,15 @@ __global__ void __launch_bounds__(kThreads, 2) k_fo(const FoArgs p) {
             const float4 wzv = dz4<N, false>(sOm + (r + SHX) * SC + scol, a, dvz);  // domegadz
             const float4 dA = dz4<N, true>(sQxx + r * SC + scol, a, dvz);           // dux_xdz = D+z Qxx
             const float4 dC = dz4<N, false>(sQzx + r * SC + scol, a, dvz);          // duz_xdz = D-z Qzx
-            const int g = gi * P + (z0 + c);
-            const float4 axv = ld4(p.ax + g), azv = ld4(p.az + g);
-            const float4 opx = ld4(p.vold[0] + g), opz = ld4(p.vold[1] + g);
-            const float4 osx = ld4(p.vold[2] + g), osz = ld4(p.vold[3] + g);
-            float4 npx, npz, nsx, nsz;
-            const bool row_live = gi >= N && gi < p.X - N;
-            const bool flat = undamped4(axv, azv);
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                const int gj = z0 + c + k;
-                const bool live = row_live && gj >= N && gj < p.Z - N;
-                const float C = comp(dC, k), E = comp(dE[0], k), A = comp(dA, k), B = comp(dB[0], k);
-                const float sum_px = __fsub_rn(__fadd_rn(comp(txv[0], k), C), E);
-                const float sum_pz = __fsub_rn(__fadd_rn(comp(tzv, k), B), A);
-                const float sum_sx = __fsub_rn(__fadd_rn(comp(wzv, k), C), E);
-                const float sum_sz = __fsub_rn(__fadd_rn(-comp(wxv[0], k), B), A);
-                float vpx, vpz, vsx, vsz;
-                if (flat) {
-                    vpx = __fadd_rn(comp(opx, k), __fmul_rn(dt, sum_px));
-                    vpz = __fadd_rn(comp(opz, k), __fmul_rn(dt, sum_pz));
-                    vsx = __fadd_rn(comp(osx, k), __fmul_rn(dt, sum_sx));
-                    vsz = __fadd_rn(comp(osz, k), __fmul_rn(dt, sum_sz));
-                } else {
-                    const float dax = comp(axv, k), daz = comp(azv, k);
-                    vpx = vel_upd(dax, dt, comp(opx, k), sum_px);
-                    vpz = vel_upd(daz, dt, comp(opz, k), sum_pz);
-                    vsx = vel_upd(dax, dt, comp(osx, k), sum_sx);
-                    vsz = vel_upd(daz, dt, comp(osz, k), sum_sz);
-                }
-                if (!live) vpx = vpz = vsx = vsz = 0.f;
-                set_comp(npx, k, vpx); set_comp(npz, k, vpz); set_comp(nsx, k, vsx); set_comp(nsz, k, vsz);
-            }
-            st4(p.vnew[0] + g, npx); st4(p.vnew[1] + g, npz);
-            st4(p.vnew[2] + g, nsx); st4(p.vnew[3] + g, nsz);
+            const bool flat = !damped || undamped4(axv, azv);
+            const unsigned live = fo_live(p, N, gi, z0 + c);
+            float4 npx = fo_vel4(flat, axv, dt, opx, sub4(add4(txv[0], dC), dE[0]));
+            float4 npz = fo_vel4(flat, azv, dt, opz, sub4(add4(tzv, dB[0]), dA));
+            float4 nsx = fo_vel4(flat, axv, dt, osx, sub4(add4(wzv, dC), dE[0]));
+            float4 nsz = fo_vel4(flat, azv, dt, osz, sub4(add4(neg4(wxv[0]), dB[0]), dA));
+            if (live != 0xfu) { npx = fo_mask(npx, live); npz = fo_mask(npz, live); nsx = fo_mask(nsx, live); nsz = fo_mask(nsz, live); }
+            stg4(p.vnew[0] + g, npx); stg4(p.vnew[1] + g, npz);
+            stg4(p.vnew[2] + g, nsx); stg4(p.vnew[3] + g, nsz);
             if (p.rec_x && p.rz >= z0 + c && p.rz < z0 + c + 4 && gi < p.X) {
                 const int k = p.rz - z0 - c;   // post-update value at the receiver row
                 p.rec_x[gi] = comp(npx, k) + comp(nsx, k);
@@ -266,16 +318,217 @@ __global__ void __launch_bounds__(kThreads, 2) k_fo(const FoArgs p) {
     }
 }
 
+// The same step on small tiles, its work cut across threads as in
+// fd_small.cuh: the x-damped stresses (theta_x, omega_x, Qxx, Qzx) need only
+// the two x derivatives and the z-damped ones only the two z derivatives, so
+// an item's x and z threads meet only in theta and omega; four threads per U
+// item take two stress derivatives each and finish one velocity component.
+template <int N, int TXr, int CTAS>
+__global__ void __launch_bounds__(SmallGeo<N, TXr>::NT, CTAS) k_fo_small(const __grid_constant__ FoArgs p) {
+    using G = SmallGeo<N, TXr>;
+    constexpr int TX = G::TX, TZ = G::TZ, SHX = G::SHX, HS = G::HS, HU = G::HU, UC = G::UC, SC = G::SC, NT = G::NT;
+    extern __shared__ __align__(128) float4 smem4[];
+    float* sm = reinterpret_cast<float*>(smem4);
+    float* sUx = sm + G::oUx;
+    float* sUz = sm + G::oUz;
+    float* sTh = sm + G::oTh;
+    float* sOm = sm + G::oOm;
+    float* sQxz = sm + G::oQxz;
+    float* sQzz = sm + G::oQzz;
+    float* sQxx = sm + G::oQxx;
+    float* sQzx = sm + G::oQzx;
+    float4* const sE = reinterpret_cast<float4*>(sm + G::oE);       // [2][itemsS]: theta_z, omega_z
+    float4* const sD = reinterpret_cast<float4*>(sm);               // [8][itemsU]: derivatives
+    float4* const sN = reinterpret_cast<float4*>(sm + G::oNew);     // [4][itemsU]: new velocities
+    __shared__ uint64_t bar;
+    const int tid = threadIdx.x;
+    const int P = p.pitch;
+    const int tz = blockIdx.x % p.tiles_z, tx = blockIdx.x / p.tiles_z;
+    const int x0 = tx * TX, z0 = tz * TZ;
+    pdl_launch_dependents();
+    if (tid == 0) {
+        mbar_init(&bar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+        prefetch_map(&p.map);
+    }
+    float a[N];
+#pragma unroll
+    for (int k = 0; k < N; ++k) a[k] = p.a[k];
+    const Div dvx = make_div(p.dx, p.rdx), dvz = make_div(p.dz, p.rdz);
+    const float dt = p.dt;
+    const bool damped = fo_damped<G>(p, x0, z0);
+    const bool xt = tid < NT / 2;   // x thread of an S item, or z thread
+    const int item = xt ? tid : tid - NT / 2;
+    const bool has_s = item < G::itemsS;
+    int r = 0, c = 0;
+    if (has_s) {
+        if (item < G::itemsA) {
+            r = -SHX + item / (TZ / 4);
+            c = 4 * (item % (TZ / 4));
+        } else {
+            const int k = item - G::itemsA, cc = k % (2 * HS / 4);
+            r = k / (2 * HS / 4);
+            c = cc < HS / 4 ? -HS + 4 * cc : TZ + 4 * (cc - HS / 4);
+        }
+    }
+    const int gs = (x0 + r) * P + (z0 + c);
+    const int task = tid / G::itemsU, ui = tid % G::itemsU;   // theta omega | Qxz Qzz along x, theta omega | Qxx Qzx along z
+    const bool has_u = task < 4;
+    const int ur = ui / (TZ / 4), uc = 4 * (ui % (TZ / 4));
+    const int gi = x0 + ur, gu = gi * P + (z0 + uc);
+    float4 vp2v = zero4(), vs2v = zero4(), axs = zero4(), azs = zero4(), so[4];
+    if (has_s) {
+        vp2v = ldg4(p.vp2 + gs);
+        vs2v = ldg4(p.vs2 + gs);
+        if (damped) { axs = ldg4(p.ax + gs); azs = ldg4(p.az + gs); }
+    }
+    __syncthreads();   // the mbarrier is initialised
+    pdl_wait();
+    if (tid == 0) issue_box<G>(&p.map, p.vfield, 0u, sm, x0, z0, 0, &bar);
+    if (has_s) {
+        // theta_x omega_x Qxx Qzx | theta_z omega_z Qxz Qzz
+#pragma unroll
+        for (int f = 0; f < 4; ++f) so[f] = ldg4((xt ? p.sold[2 * f] : p.sold[2 * f + 1]) + gs);
+    }
+    if (!fo_u_box<G>(p, sm, x0, z0, &bar)) return;
+
+    // ---- stresses ------------------------------------------------------------
+    const float* ux0 = sUx + (r + SHX + N) * UC + (c + HU);
+    const float* uz0 = sUz + (r + SHX + N) * UC + (c + HU);
+    const int sr = r + SHX, scol = c + HS;
+    float4 v0 = zero4(), v1 = zero4();   // theta_x, omega_x of an x thread
+    unsigned slive = 0;
+    if (has_s) {
+        const bool flat = !damped || undamped4(axs, azs);
+        const float4 cp = mul4s(vp2v, dt), cs = mul4s(vs2v, dt);
+        slive = fo_live(p, N, x0 + r, z0 + c);
+        float4 d1, d2;   // exx, ezx | ezz, exz
+        if (xt) {
+            float4 e1[1], e2[1];
+            dx4<N, 1, false>(ux0, UC, a, dvx, e1);   // dvxdx = D-x Vx
+            dx4<N, 1, true>(uz0, UC, a, dvx, e2);    // dvzdx = D+x Vz
+            d1 = e1[0];
+            d2 = e2[0];
+        } else {
+            d2 = dz4<N, true>(ux0, a, dvz);    // dvxdz = D+z Vx
+            d1 = dz4<N, false>(uz0, a, dvz);   // dvzdz = D-z Vz
+        }
+        const float4 dd = xt ? axs : azs;
+        v0 = fo_stress4(flat, dd, dt, prod4(cp, d1), so[0]);                     // theta_x | theta_z
+        v1 = fo_stress4(flat, dd, dt, prod4(xt ? neg4(cs) : cs, d2), so[1]);     // omega_x | omega_z
+        float4 v2 = fo_stress4(flat, dd, dt, prod4(cs, xt ? d1 : d2), so[2]);    // Qxx | Qxz
+        float4 v3 = fo_stress4(flat, dd, dt, prod4(cs, xt ? d2 : d1), so[3]);    // Qzx | Qzz
+        if (slive != 0xfu) { v0 = fo_mask(v0, slive); v1 = fo_mask(v1, slive); v2 = fo_mask(v2, slive); v3 = fo_mask(v3, slive); }
+        if (r >= 0 && r < TX && c >= 0 && c < TZ) {
+            const float4 v[4] = {v0, v1, v2, v3};
+#pragma unroll
+            for (int f = 0; f < 4; ++f) stg4((xt ? p.snew[2 * f] : p.snew[2 * f + 1]) + gs, v[f]);
+        }
+        if (xt) {
+            if (r >= 0 && r < TX) {
+                st4(sQxx + r * SC + scol, v2);
+                st4(sQzx + r * SC + scol, v3);
+            }
+        } else {
+            sE[item] = v0;
+            sE[G::itemsS + item] = v1;
+            if (item < G::itemsA) {
+                st4(sQxz + sr * TZ + c, v2);
+                st4(sQzz + sr * TZ + c, v3);
+            }
+        }
+    }
+    float4 old = zero4(), dd = zero4(), ax2 = zero4(), az2 = zero4();   // U operands
+    if (has_u) {
+        old = ldg4((task == 0 ? p.vold[0] : task == 1 ? p.vold[1] : task == 2 ? p.vold[2] : p.vold[3]) + gu);
+        if (damped) { ax2 = ldg4(p.ax + gu); az2 = ldg4(p.az + gu); }
+    }
+    __syncthreads();
+    if (has_s && xt) {
+        float4 sv = zero4();
+        const int k = p.sz - z0 - c;
+        if (p.wavelet && x0 + r == p.sx && k >= 0 && k < 4 && (slive >> k & 1u)) set_comp(sv, k, p.wavelet[p.t]);
+        st4(sTh + sr * SC + scol, add4(add4(v0, sE[item]), sv));   // PS:557
+        st4(sOm + sr * SC + scol, add4(v1, sE[G::itemsS + item]));
+    }
+    __syncthreads();
+
+    // ---- velocities ------------------------------------------------------------
+    if (has_u) {
+        float4 d1, d2;
+        if (task < 2) {
+            float4 e1[1], e2[1];
+            if (task == 0) {
+                dx4<N, 1, true>(sTh + (ur + SHX) * SC + (uc + HS), SC, a, dvx, e1);    // dthetadx
+                dx4<N, 1, false>(sOm + (ur + SHX) * SC + (uc + HS), SC, a, dvx, e2);   // domegadx
+            } else {
+                dx4<N, 1, false>(sQxz + (ur + SHX) * TZ + uc, TZ, a, dvx, e1);         // dux_zdx = B
+                dx4<N, 1, true>(sQzz + (ur + SHX) * TZ + uc, TZ, a, dvx, e2);          // duz_zdx = E
+            }
+            d1 = e1[0];
+            d2 = e2[0];
+        } else {
+            const float* f1 = task == 2 ? sTh + (ur + SHX) * SC + (uc + HS) : sQxx + ur * SC + (uc + HS);
+            const float* f2 = task == 2 ? sOm + (ur + SHX) * SC + (uc + HS) : sQzx + ur * SC + (uc + HS);
+            d1 = dz4<N, true>(f1, a, dvz);    // dthetadz | dux_xdz = A
+            d2 = dz4<N, false>(f2, a, dvz);   // domegadz | duz_xdz = C
+        }
+        sD[(2 * task) * G::itemsU + ui] = d1;
+        sD[(2 * task + 1) * G::itemsU + ui] = d2;
+    }
+    __syncthreads();
+    if (has_u) {
+        auto D = [&](int k) { return sD[k * G::itemsU + ui]; };   // tx wx B E tz wz A C
+        const bool xc = task == 0 || task == 2;
+        float4 e0 = D(task == 0 ? 0 : task == 1 ? 4 : task == 2 ? 5 : 1);
+        if (task == 3) e0 = neg4(e0);
+        const float4 sum = sub4(add4(e0, xc ? D(7) : D(2)), xc ? D(3) : D(6));
+        const bool flat = !damped || undamped4(ax2, az2);
+        dd = xc ? ax2 : az2;
+        float4 nv = fo_vel4(flat, dd, dt, old, sum);
+        const unsigned live = fo_live(p, N, gi, z0 + uc);
+        if (live != 0xfu) nv = fo_mask(nv, live);
+        stg4((task == 0 ? p.vnew[0] : task == 1 ? p.vnew[1] : task == 2 ? p.vnew[2] : p.vnew[3]) + gu, nv);
+        sN[task * G::itemsU + ui] = nv;
+    }
+    if (p.rec_x && p.rz >= z0 && p.rz < z0 + TZ) {
+        __syncthreads();
+        if (tid < TX && x0 + tid < p.X) {
+            const float* n0 = sm + G::oNew;
+            const int o = tid * TZ + (p.rz - z0);
+            p.rec_x[x0 + tid] = n0[o] + n0[2 * TX * TZ + o];   // post-update value at the receiver row
+            p.rec_z[x0 + tid] = n0[TX * TZ + o] + n0[3 * TX * TZ + o];
+        }
+    }
+}
+
 // The shared-memory opt-in is a per-device attribute: set on the current
 // device before every loop (fo_run), not once per process.
 template <int N>
 cudaError_t configure() {
-    return cudaFuncSetAttribute(k_fo<N>, cudaFuncAttributeMaxDynamicSharedMemorySize, TileGeo<N>::bytes);
+    auto set = [](auto kernel, int bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+    };
+    cudaError_t e = set(k_fo<N, TileGeo<N>>, TileGeo<N>::bytes);
+    if (e == cudaSuccess) e = set(k_fo<N, MidGeo<N>>, MidGeo<N>::bytes);
+    if (e == cudaSuccess) e = set(k_fo_small<N, 16, 1>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = set(k_fo_small<N, 16, 2>, SmallGeo<N, 16>::bytes);
+    if (e == cudaSuccess) e = set(k_fo_small<N, 24, 1>, SmallGeo<N, 24>::bytes);
+    return e;
 }
 
+// One step on the tiles of `tier` (pick_tier: the same shapes pay at the same
+// sizes as for the second-order step).
 template <int N>
-void launch(const FoArgs& a, int tiles_x, cudaStream_t s) {
-    k_fo<N><<<tiles_x * a.tiles_z, kThreads, TileGeo<N>::bytes, s>>>(a);
+void launch(FoArgs& a, Tier tier, cudaStream_t s) {
+    const int tx = tier == kLarge ? 32 : tier == kSmall24 ? 24 : 16, tz = tier == kLarge || tier == kMid ? 64 : 32;
+    a.tiles_z = (a.Z + tz - 1) / tz;
+    const dim3 grid((a.X + tx - 1) / tx * a.tiles_z);
+    if (tier == kLarge) launch_pdl(k_fo<N, TileGeo<N>>, grid, kThreads, TileGeo<N>::bytes, s, a);
+    else if (tier == kMid) launch_pdl(k_fo<N, MidGeo<N>>, grid, kThreads, MidGeo<N>::bytes, s, a);
+    else if (tier == kSmall24) launch_pdl(k_fo_small<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, a);
+    else if (tier == kSmall16) launch_pdl(k_fo_small<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a);
+    else launch_pdl(k_fo_small<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a);
 }
 
 // Five-digit weights of the reference's first-order kernels (PS:405,
@@ -340,13 +593,18 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     a.rdx = 1.0f / ctx->cfg.dx; a.rdz = 1.0f / ctx->cfg.dz;
     a.vp2 = ctx->field(ctx->fo_sq, 0); a.vs2 = ctx->field(ctx->fo_sq, 1); a.ax = ctx->ax; a.az = ctx->az;
     a.wavelet = backward ? nullptr : ctx->d_wavelet;
+    a.err = ctx->d_status;
+    const StepArgs b = base_args(ctx);
+    const Tier tier = pick_tier(ctx->N, nullptr, &b, kFwd, 1);
+    a.map = tier == kLarge ? b.box_map : tier == kMid ? b.mid_map : b.small_map[tier == kSmall24 ? 1 : 0];
+    auto field_of = [&](const float* f) { return (int)((f - ctx->field(ctx->state, 0)) / (ptrdiff_t)ctx->fstride); };
     float* gx = ctx->gather(0, 0);
     float* gz = ctx->gather(0, 1);
     cudaEventRecord(ctx->ev[1], ctx->stream);
     for (int n = 0; n < ctx->nt; ++n) {
         const int t = backward ? ctx->nt - 1 - n : n;
         const bool even = (n & 1) == 0;
-        for (int k = 0; k < 4; ++k) { a.vold[k] = even ? vA[k] : vB[k]; a.vnew[k] = even ? vB[k] : (float*)vA[k]; }
+        for (int k = 0; k < 4; ++k) { a.vold[k] = even ? vA[k] : vB[k]; a.vnew[k] = even ? vB[k] : (float*)vA[k]; a.vfield[k] = field_of(a.vold[k]); }
         for (int k = 0; k < 8; ++k) { a.sold[k] = even ? sA[k] : sB[k]; a.snew[k] = even ? sB[k] : sA[k]; }
         a.t = t;
         if (backward) {
@@ -356,9 +614,9 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
             a.rec_x = gx + (size_t)t * ctx->X;
             a.rec_z = gz + (size_t)t * ctx->X;
         }
-        if (ctx->N == 2) fo::launch<2>(a, ctx->tiles_x, ctx->stream);
-        else if (ctx->N == 5) fo::launch<5>(a, ctx->tiles_x, ctx->stream);
-        else fo::launch<6>(a, ctx->tiles_x, ctx->stream);
+        if (ctx->N == 2) fo::launch<2>(a, tier, ctx->stream);
+        else if (ctx->N == 5) fo::launch<5>(a, tier, ctx->stream);
+        else fo::launch<6>(a, tier, ctx->stream);
         ctx->timing.kernel_launches += 1;
     }
     cudaEventRecord(ctx->ev[2], ctx->stream);
@@ -385,6 +643,7 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     }
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "first-order time loop");
+    if ((rc = check_status(ctx))) return rc;
     if (fields) {
         // totals as the kernels form them: U = P + S, theta = theta_x + theta_z + s,
         // omega = omega_x + omega_z

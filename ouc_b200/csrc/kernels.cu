@@ -60,23 +60,6 @@ int march_segments(Mode mode, const StepArgs& a) {
     return (row_end - row0 + a.seg_rows - 1) / a.seg_rows;
 }
 
-// Launch with programmatic stream serialization: the kernel may start before
-// the launch ahead of it in the stream has finished (pdl_wait orders them).
-template <class... P, class... A>
-static void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, const A&... args) {
-    cudaLaunchAttribute at[1];
-    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    at[0].val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t c = {};
-    c.gridDim = grid;
-    c.blockDim = dim3(threads);
-    c.dynamicSmemBytes = smem;
-    c.stream = s;
-    c.attrs = at;
-    c.numAttrs = 1;
-    cudaLaunchKernelEx(&c, kernel, args...);
-}
-
 struct Grid {
     int tiles_z, tiles;
 };
