@@ -517,21 +517,13 @@ int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src) {
         CK(cudaGetLastError());
         return OUC_OK;
     }
-    if (ctx->cfg.gradient || !ctx->stream2) {
-        for (int t = ctx->nt - 1; t >= 0; --t) {
-            if ((rc = rcv_step(ctx, ar, r, n, t))) return rc;
-            if (ctx->cfg.gradient) grad_step(ctx, s, r, n, t);
-            if ((rc = rec_step(ctx, as, s, r, n, t, exact_strips, theta_src))) return rc;
-        }
-        CK(cudaGetLastError());
-        return OUC_OK;
-    }
     // Two streams, so that the reconstruction of step t overlaps the
     // receiver step t-1: rec(t) reads the receiver level rcv(t) wrote and
     // rcv(t-1) only reads it too (it writes the older buffer), so the two are
     // independent; rcv(t-2) overwrites that level and waits for rec(t).  The
-    // source side stays in order on the context stream.  Same launches, same
-    // arguments, same results as the serial loop.
+    // source side stays in order on the context stream, the gradient's
+    // correlation of step t ahead of rec(t).  Same launches, same arguments,
+    // same results as the serial loop.
     cudaStream_t sr = ctx->stream2;
     CK(cudaEventRecord(ctx->evb[0], ctx->stream));   // the receiver stream starts after the work queued so far
     CK(cudaStreamWaitEvent(sr, ctx->evb[0], 0));
@@ -540,6 +532,7 @@ int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src) {
         if ((rc = rcv_step(ctx, ar, r, n, t, sr))) return rc;
         CK(cudaEventRecord(ctx->evb[0], sr));
         CK(cudaStreamWaitEvent(ctx->stream, ctx->evb[0], 0));                          // rcv(t) is done
+        if (ctx->cfg.gradient) grad_step(ctx, s, r, n, t);   // reads both sides as rec(t) does, before it
         if ((rc = rec_step(ctx, as, s, r, n, t, exact_strips, theta_src))) return rc;
         CK(cudaEventRecord(ctx->evb[1 + (t & 1)], ctx->stream));
     }
@@ -937,7 +930,7 @@ int ouc_destroy(ouc_ctx* ctx) {
     for (auto* p : ctx->d_stack) cudaFree(p);
     cudaFree(ctx->strips); cudaFree(ctx->stage); cudaFree(ctx->amax);
     cudaFree(ctx->snaps); cudaFree(ctx->snap_amax);
-    cudaFree(ctx->l_in); cudaFree(ctx->l_out); cudaFree(ctx->l_truth); cudaFree(ctx->l_scale); cudaFree(ctx->l_tmp); cudaFree(ctx->sv_model);
+    cudaFree(ctx->l_in); cudaFree(ctx->l_out); cudaFree(ctx->l_truth); cudaFree(ctx->l_scale); cudaFree(ctx->l_tmp); cudaFree(ctx->sv_model); cudaFree(ctx->sv_pow4);
     cudaFree(ctx->grad); cudaFree(ctx->fo_sq);
     for (auto* p : ctx->d_gstack) cudaFree(p);
     for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.exec);

@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstring>
 #include <string>
 #include <vector>
@@ -40,7 +41,36 @@ float* slot_field(const ouc_ctx* c, int b, int k) {
     return c->sv_model + ((size_t)b * kModelFields + k) * c->fstride + (size_t)kGX * c->pitch + kZOFF;
 }
 
+// Damping profile of a window's own edges (host::damping, PS:2067-2105) from
+// the padded Vp on the device: the same double products in the same order,
+// with the fourth powers of k / L tabulated on the host.  Bound by its writes
+// (two fields of the window); on the host the powers of every damped cell and
+// the upload took about 7 ms for a window of 1000 x 860 cells.
+__global__ void k_window_damping(const float* __restrict__ vp, int X, int Z, int L, int pitch, double g,
+                                 const double* __restrict__ pow4, float* ax, float* az) {
+    const int i = blockIdx.y;
+    for (int j = threadIdx.x + blockIdx.x * blockDim.x; j < Z; j += blockDim.x * gridDim.x) {
+        const ptrdiff_t c = (ptrdiff_t)i * pitch + j;
+        const int kx = i < L ? L - i : i > X - L ? i - X + L : 0, kz = j < L ? L - j : j > Z - L ? j - Z + L : 0;
+        const double s = __ddiv_rn(__dmul_rn(g, (double)vp[c]), (double)L);
+        ax[c] = kx ? (float)__dmul_rn(s, pow4[kx]) : 0.f;
+        az[c] = kz ? (float)__dmul_rn(s, pow4[kz]) : 0.f;
+    }
+}
+
 int ensure_model(ouc_ctx* ctx) {
+    if (!ctx->sv_pow4) {
+        std::vector<double> t(ctx->L + 1);
+        for (int k = 0; k <= ctx->L; ++k) t[k] = pow(1.0 * k / ctx->L, 4.0);
+        if (cudaMalloc(&ctx->sv_pow4, t.size() * sizeof(double)) != cudaSuccess) {
+            cudaGetLastError();
+            ctx->sv_pow4 = nullptr;
+            return fail(ctx, OUC_ENOMEM, "cannot allocate the sub-grid models");
+        }
+        CKS(cudaMemcpyAsync(ctx->sv_pow4, t.data(), t.size() * sizeof(double), cudaMemcpyHostToDevice, ctx->stream));
+        CKS(cudaStreamSynchronize(ctx->stream));
+        ctx->bytes += t.size() * sizeof(double);
+    }
     if (ctx->sv_model) return OUC_OK;
     const size_t bytes = (size_t)ctx->batch * kModelFields * ctx->fstride * sizeof(float);
     if (cudaMalloc(&ctx->sv_model, bytes) != cudaSuccess) {
@@ -71,10 +101,8 @@ int check(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap) {
     return OUC_OK;
 }
 
-// Descriptors and sub-grid models of one batch; `keep` holds the host
-// damping arrays until the batch's final synchronisation.
-int upload_batch(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, const float* d_w,
-                 std::vector<std::vector<float>>& keep) {
+// Descriptors and sub-grid models of one batch.
+int upload_batch(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, const float* d_w) {
     int rc = ensure_model(ctx);
     if (rc) return rc;
     const int L = ctx->L, Z = ctx->Z, TX = 32, pitch = ctx->pitch;
@@ -92,16 +120,10 @@ int upload_batch(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture*
         }
         // damping profile of the window's own edges (the profile a context
         // created on this window as a padded model computes)
-        std::vector<float> vpw(ctx->vp_host.begin() + (size_t)w.x0 * Z, ctx->vp_host.begin() + (size_t)(w.x0 + w.X) * Z);
-        keep.emplace_back((size_t)w.X * Z);
-        keep.emplace_back((size_t)w.X * Z);
-        std::vector<float>& ax = keep[keep.size() - 2];
-        std::vector<float>& az = keep[keep.size() - 1];
-        damping(vpw, w.X, Z, L, ctx->cfg.pml_r, ax, az);
-        CKS(cudaMemcpy2DAsync(slot_field(ctx, b, 2), (size_t)pitch * 4, ax.data(), (size_t)Z * 4, (size_t)Z * 4, w.X,
-                              cudaMemcpyHostToDevice, ctx->stream));
-        CKS(cudaMemcpy2DAsync(slot_field(ctx, b, 3), (size_t)pitch * 4, az.data(), (size_t)Z * 4, (size_t)Z * 4, w.X,
-                              cudaMemcpyHostToDevice, ctx->stream));
+        k_window_damping<<<dim3((Z + 255) / 256, w.X), 256, 0, ctx->stream>>>(
+            ctx->vpv + (size_t)w.x0 * pitch, w.X, Z, L, pitch, log10(1.0 / ctx->cfg.pml_r) * 1.5, ctx->sv_pow4,
+            slot_field(ctx, b, 2), slot_field(ctx, b, 3));
+        ctx->timing.kernel_launches += 1;
         ShotDesc& s = d[b];
         memset(&s, 0, sizeof(s));
         s.sx = shots[b].sx - w.x0 + L;
@@ -158,8 +180,7 @@ int gather_to_host(ouc_ctx* ctx, const float* src_tx, float* dst, int Xb) {
 int group(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, const float* d_w, bool forward_only,
           float* const* gx, float* const* gz, const float* const* rx, const float* const* rz, float* const* ipp,
           float* const* ips) {
-    std::vector<std::vector<float>> keep;
-    int rc = upload_batch(ctx, n, shots, ap, d_w, keep);
+    int rc = upload_batch(ctx, n, shots, ap, d_w);
     if (rc) return rc;
     const bool self_records = !forward_only && rx == nullptr;
     CKS(cudaEventRecord(ctx->ev[0], ctx->stream));
