@@ -464,6 +464,7 @@ void grad_step(ouc_ctx* ctx, const Side& s, const Side& r, int n, int t) {
     g.nshots = n;
     for (int k = 0; k < 6; ++k) g.a[k] = ctx->a[k];
     g.dx = ctx->cfg.dx; g.dz = ctx->cfg.dz;
+    g.rdx = 1.0f / ctx->cfg.dx; g.rdz = 1.0f / ctx->cfg.dz;
     const bool past = t < ctx->nt - 1 && ctx->cfg.image_align == OUC_IMAGE_REFERENCE;
     for (int k = 0; k < 4; ++k) { g.src[k] = past ? s.past[k] : s.now[k]; g.rcv[k] = r.now[k]; }
     g.shot_stride = ctx->shot_stride;

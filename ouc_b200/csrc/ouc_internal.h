@@ -258,7 +258,7 @@ struct GradArgs {
     int X, Z, pitch, L, N;
     int nshots;
     float a[6];
-    float dx, dz;
+    float dx, dz, rdx, rdz;  // spacings and RN(1 / spacing)
     const float* src[4];     // source Px Pz Sx Sz at the imaged level (shot 0)
     const float* rcv[4];     // receiver Px Pz Sx Sz after the back-step (shot 0)
     size_t shot_stride;      // state floats between shots
