@@ -587,24 +587,6 @@ int finalize(ouc_ctx* ctx, int n) {
     return OUC_OK;
 }
 
-// Bring a gather from the caller's layout into the time-major device gather.
-int gather_in(ouc_ctx* ctx, const float* src, float* dst_tx, bool host) {
-    const size_t n = (size_t)ctx->nt * ctx->X;
-    const bool xt = ctx->cfg.gather_layout == OUC_GATHER_XT;
-    if (!xt) {
-        CK(cudaMemcpyAsync(dst_tx, src, n * 4, host ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToDevice, ctx->stream));
-        return OUC_OK;
-    }
-    const float* from = src;
-    if (host) {
-        CK(cudaMemcpyAsync(ctx->staging, src, n * 4, cudaMemcpyHostToDevice, ctx->stream));
-        from = ctx->staging;
-    }
-    launch_transpose(from, dst_tx, ctx->X, ctx->nt, ctx->stream);   // [X][nt] -> [nt][X]
-    ctx->timing.kernel_launches += 1;
-    return OUC_OK;
-}
-
 int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host) {
     const size_t n = (size_t)ctx->nt * ctx->X;
     const bool xt = ctx->cfg.gather_layout == OUC_GATHER_XT;
@@ -616,8 +598,21 @@ int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host) {
         from = tgt;
         if (!host) return OUC_OK;
     }
-    CK(cudaMemcpyAsync(dst, from, n * 4, host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice, ctx->stream));
+    if (host) return to_host(ctx, dst, from, n * 4);
+    CK(cudaMemcpyAsync(dst, from, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     return OUC_OK;
+}
+
+int fields_out(ouc_ctx* ctx, const Side& s, float* fields) {
+    const float* f[4] = {s.now[0], s.now[1], s.now[2], s.now[3]};
+    const size_t C = (size_t)ctx->X * ctx->Z;
+    int rc;
+    touch_pages({{fields, nullptr, 6 * C * 4}});   // while the time loop runs
+    launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
+    if ((rc = to_host(ctx, fields + 2 * C, ctx->staging, 4 * C * 4))) return rc;
+    launch_pack_fields(f, 2, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream, f + 2);   // P + S
+    CK(cudaGetLastError());
+    return to_host(ctx, fields, ctx->staging, 2 * C * 4);
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -839,6 +834,7 @@ int ouc_create(const ouc_config* cfg, const float* vp, const float* vs, const fl
     const size_t ng = (size_t)ctx->nt * X;
     const size_t ni = (size_t)ctx->nx * ctx->nz;
     const size_t stage = std::max(ng, (size_t)4 * X * Z);
+    ctx->staging_n = stage;
     bool ok = cudaMalloc(&ctx->model, model_bytes) == cudaSuccess &&
               cudaMalloc(&ctx->state, state_bytes) == cudaSuccess &&
               cudaMalloc(&ctx->gathers, 2 * ng * ctx->batch * 4) == cudaSuccess &&
@@ -924,6 +920,7 @@ int ouc_create(const ouc_config* cfg, const float* vp, const float* vs, const fl
 int ouc_destroy(ouc_ctx* ctx) {
     if (!ctx) return OUC_OK;
     if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    free_ring(ctx);
     cudaFree(ctx->model); cudaFree(ctx->state);
     cudaFree(ctx->gathers); cudaFree(ctx->staging); cudaFree(ctx->d_wavelet);
     cudaFree(ctx->d_img); cudaFree(ctx->d_desc); cudaFree(ctx->d_status);
@@ -1043,22 +1040,10 @@ static int forward_impl(ouc_ctx* ctx, const ouc_shot* shot, const float* wavelet
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
     if (gx && (rc = gather_out(ctx, ctx->gather(0, 0), gx, host))) return rc;
     if (gz && (rc = gather_out(ctx, ctx->gather(0, 1), gz, host))) return rc;
-    if (fields && host) {
-        const float* f[4] = {ctx->src.now[0], ctx->src.now[1], ctx->src.now[2], ctx->src.now[3]};
-        launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
-        const size_t C = (size_t)ctx->X * ctx->Z;
-        CK(cudaMemcpyAsync(fields + 2 * C, ctx->staging, 4 * C * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    }
+    if (fields && host && (rc = fields_out(ctx, ctx->src, fields))) return rc;
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
-    if (fields && host) {
-        const size_t C = (size_t)ctx->X * ctx->Z;
-        for (size_t k = 0; k < C; ++k) {
-            fields[k] = fields[2 * C + k] + fields[4 * C + k];       // Ux = Px + Sx
-            fields[C + k] = fields[3 * C + k] + fields[5 * C + k];   // Uz = Pz + Sz
-        }
-    }
     ctx->timing.forward_ms = elapsed(ctx->ev[1], ctx->ev[2]);
     ctx->timing.copy_ms = elapsed(ctx->ev[0], ctx->ev[1]) + elapsed(ctx->ev[2], ctx->ev[3]);
     return OUC_OK;
@@ -1080,12 +1065,15 @@ static int rtm_group(ouc_ctx* ctx, int n, const ouc_shot* shots, const float* d_
     const bool snap = ctx->cfg.snapshot_every > 0;
     if ((rc = upload_desc(ctx, n, shots, d_w))) return rc;
     CK(cudaEventRecord(ctx->ev[0], ctx->stream));
+    if (!self_records && (rc = records_fence(ctx))) return rc;
     if ((rc = run_forward(ctx, n, self_records, !snap, snap))) return rc;
+    std::vector<Record> recs;
     for (int b = 0; b < n && !self_records; ++b) {
         if (!rx[b] || !rz[b]) return fail(ctx, OUC_EINVAL, "record pointer missing for a shot");
-        if ((rc = gather_in(ctx, rx[b], ctx->gather(b, 0), host))) return rc;
-        if ((rc = gather_in(ctx, rz[b], ctx->gather(b, 1), host))) return rc;
+        recs.push_back({rx[b], ctx->gather(b, 0), ctx->X});
+        recs.push_back({rz[b], ctx->gather(b, 1), ctx->X});
     }
+    if ((rc = records_beside(ctx, recs, host))) return rc;
     for (int b = 0; b < n; ++b) {
         if (!shots[b].mute) continue;
         const int sx = shots[b].sx + ctx->L, sz = shots[b].sz + ctx->L, rzz = shots[b].rz + ctx->L;
@@ -1120,11 +1108,16 @@ static int rtm_group(ouc_ctx* ctx, int n, const ouc_shot* shots, const float* d_
         ctx->timing.kernel_launches += 1;
     }
     const size_t ni = (size_t)ctx->nx * ctx->nz;
-    const cudaMemcpyKind kind = host ? cudaMemcpyDeviceToHost : cudaMemcpyDeviceToDevice;
-    for (int b = 0; b < n; ++b) {
-        if (ipp && ipp[b]) CK(cudaMemcpyAsync(ipp[b], ctx->d_img + (size_t)(2 * b) * ni, ni * 4, kind, ctx->stream));
-        if (ips && ips[b]) CK(cudaMemcpyAsync(ips[b], ctx->d_img + (size_t)(2 * b + 1) * ni, ni * 4, kind, ctx->stream));
-    }
+    std::vector<HostCopy> images;
+    for (int b = 0; b < n; ++b)
+        for (int k = 0; k < 2; ++k) {
+            float* dst = k == 0 ? (ipp ? ipp[b] : nullptr) : (ips ? ips[b] : nullptr);
+            float* src = ctx->d_img + (size_t)(2 * b + k) * ni;
+            if (!dst) continue;
+            if (host) images.push_back({dst, src, ni * 4});
+            else CK(cudaMemcpyAsync(dst, src, ni * 4, cudaMemcpyDeviceToDevice, ctx->stream));
+        }
+    if ((rc = copy_host(ctx, images, true))) return rc;
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
@@ -1189,8 +1182,10 @@ int ouc_stack(ouc_ctx* ctx, double* pp, double* ps, double* illum, int reset) {
     cudaSetDevice(ctx->device);
     const size_t ni = (size_t)ctx->nx * ctx->nz;
     double* outs[3] = {pp, ps, illum};
+    std::vector<HostCopy> copies;
     for (int k = 0; k < 3; ++k)
-        if (outs[k]) CK(cudaMemcpyAsync(outs[k], ctx->d_stack[k], ni * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        if (outs[k]) copies.push_back({outs[k], ctx->d_stack[k], ni * 8});
+    if (int rc = copy_host(ctx, copies, true)) return rc;
     if (reset)
         for (int k = 0; k < 3; ++k) CK(cudaMemsetAsync(ctx->d_stack[k], 0, ni * 8, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1204,8 +1199,10 @@ int ouc_gradient(ouc_ctx* ctx, double* g_vp, double* g_vs, double* illum, int re
     cudaSetDevice(ctx->device);
     const size_t ni = (size_t)ctx->nx * ctx->nz;
     double* out[3] = {g_vp, g_vs, illum};
+    std::vector<HostCopy> copies;
     for (int k = 0; k < 3; ++k)
-        if (out[k]) CK(cudaMemcpyAsync(out[k], ctx->d_gstack[k], ni * 8, cudaMemcpyDeviceToHost, ctx->stream));
+        if (out[k]) copies.push_back({out[k], ctx->d_gstack[k], ni * 8});
+    if (int rc = copy_host(ctx, copies, true)) return rc;
     if (reset)
         for (int k = 0; k < 3; ++k) CK(cudaMemsetAsync(ctx->d_gstack[k], 0, ni * 8, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
@@ -1253,8 +1250,7 @@ int ouc_step_begin(ouc_ctx* ctx, const ouc_shot* shot, const float* wavelet, con
     if ((rc = upload_desc(ctx, 1, shot, ctx->d_wavelet))) return rc;
     if ((rc = zero_side(ctx, 1, 0, false)) || (rc = zero_side(ctx, 1, 1, true))) return rc;
     if (rec_vx) {
-        if ((rc = gather_in(ctx, rec_vx, ctx->gather(0, 0), true))) return rc;
-        if ((rc = gather_in(ctx, rec_vz, ctx->gather(0, 1), true))) return rc;
+        if ((rc = records_in(ctx, {{rec_vx, ctx->gather(0, 0), ctx->X}, {rec_vz, ctx->gather(0, 1), ctx->X}}, true))) return rc;
     }
     ctx->step_shot = *shot;
     ctx->step_fwd = base_args(ctx);
@@ -1318,8 +1314,8 @@ int ouc_image_finalize(ouc_ctx* ctx, float* img_pp, float* img_ps) {
     int rc = step_order(ctx, ouc_ctx::kFinalize, 0);
     if (rc || (rc = finalize(ctx, 1))) return rc;
     const size_t ni = (size_t)ctx->nx * ctx->nz;
-    if (img_pp) CK(cudaMemcpyAsync(img_pp, ctx->d_img, ni * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    if (img_ps) CK(cudaMemcpyAsync(img_ps, ctx->d_img + ni, ni * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    if (img_pp && (rc = to_host(ctx, img_pp, ctx->d_img, ni * 4))) return rc;
+    if (img_ps && (rc = to_host(ctx, img_ps, ctx->d_img + ni, ni * 4))) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     ctx->step_phase = ouc_ctx::kIdle;
     return OUC_OK;
@@ -1330,16 +1326,9 @@ int ouc_step_fields(ouc_ctx* ctx, int side, float* fields) {
     if (!fields || (side != 0 && side != 1)) return fail(ctx, OUC_EINVAL, "fields is NULL or side is not 0/1");
     if (ctx->step_phase == ouc_ctx::kIdle) return fail(ctx, OUC_ESTATE, "no shot is being stepped");
     cudaSetDevice(ctx->device);
-    const Side& s = side == 0 ? ctx->src : ctx->rcv;
-    const float* f[4] = {s.now[0], s.now[1], s.now[2], s.now[3]};
-    launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
-    const size_t C = (size_t)ctx->X * ctx->Z;
-    CK(cudaMemcpyAsync(fields + 2 * C, ctx->staging, 4 * C * 4, cudaMemcpyDeviceToHost, ctx->stream));
+    const int rc = fields_out(ctx, side == 0 ? ctx->src : ctx->rcv, fields);
+    if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
-    for (size_t k = 0; k < C; ++k) {
-        fields[k] = fields[2 * C + k] + fields[4 * C + k];       // Ux = Px + Sx (PS:302)
-        fields[C + k] = fields[3 * C + k] + fields[5 * C + k];   // Uz = Pz + Sz (PS:303)
-    }
     return OUC_OK;
 }
 

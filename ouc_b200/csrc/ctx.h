@@ -28,6 +28,8 @@ struct Side {
 
 }  // namespace ouc
 
+namespace ouc { struct HostRing; }   // hostio.cu
+
 struct ouc_ctx {
     using Ring = ouc::Ring;
     using Side = ouc::Side;
@@ -87,7 +89,8 @@ struct ouc_ctx {
     float* acc[3] = {nullptr, nullptr, nullptr};
     float* comp[3] = {nullptr, nullptr, nullptr};   // compensation terms of acc (compensated_image)
     float* gathers = nullptr;    // [batch][2][nt][X], time-major
-    float* staging = nullptr;    // max(nt*X, 4*X*Z) floats for transposes / packing
+    float* staging = nullptr;    // staging_n = max(nt*X, 4*X*Z) floats for transposes / packing
+    size_t staging_n = 0;
     float* d_wavelet = nullptr;
     float* d_img = nullptr;      // [batch][2][nx][nz]
     double* d_stack[3] = {nullptr, nullptr, nullptr};
@@ -113,6 +116,7 @@ struct ouc_ctx {
     double* sv_pow4 = nullptr;   // (k / L)^4, k = 0 .. L
     // first-order scheme (fo.cu): powf(Vp, 2), powf(Vs, 2) in the model layout, allocated on first use
     float* fo_sq = nullptr;
+    ouc::HostRing* io = nullptr;   // pinned ring of large host copies, made on first use
     size_t bytes = 0;
     cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
     cudaStream_t stream2 = nullptr;    // receiver steps of the overlapped backward loop
@@ -144,8 +148,39 @@ int zero_side(ouc_ctx* ctx, int n, int side, bool with_acc);
 int fwd_step(ouc_ctx* ctx, StepArgs& a, Side& s, int n, int t);
 int run_forward(ouc_ctx* ctx, int n, bool record, bool save, bool snaps = false);
 int run_forward_loop(ouc_ctx* ctx, int n, bool record, bool save, bool snaps);
+// Copies between device and (pageable or pinned) host memory on the context's
+// stream or `st` (hostio.cu).  As with cudaMemcpyAsync, pageable host arrays
+// may be reused on return when they are the source, and are complete after a
+// synchronisation when they are the destination.
+struct HostCopy {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st = nullptr);
+inline int to_host(ouc_ctx* ctx, void* dst, const void* src, size_t bytes) {
+    return copy_host(ctx, {{dst, const_cast<void*>(src), bytes}}, true);
+}
+void free_ring(ouc_ctx* ctx);
+// Take the page faults of large host destinations ahead of their copies.
+void touch_pages(const std::vector<HostCopy>& copies);
+// Records of the caller's layout into time-major device gathers of width X,
+// on the context's stream or `st`; host: from host memory.
+struct Record {
+    const float* src;
+    float* dst_tx;
+    int X;
+};
+int records_in(ouc_ctx* ctx, const std::vector<Record>& recs, bool host, cudaStream_t st = nullptr);
+// The same beside the work queued on the context's stream since records_fence
+// (a forward pass that does not record); later work on that stream waits for
+// it, and it waits for the work before the fence (earlier readers of the
+// gathers, producers of device records).
+int records_fence(ouc_ctx* ctx);
+int records_beside(ouc_ctx* ctx, const std::vector<Record>& recs, bool host);
+// Displacement of a wavefield, (6, X, Z): Ux = P + S, Uz, Px, Pz, Sx, Sz (PS:302-303).
+int fields_out(ouc_ctx* ctx, const Side& s, float* fields);
 int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host);
-int gather_in(ouc_ctx* ctx, const float* src, float* dst_tx, bool host);
 int ensure_strips(ouc_ctx* ctx);
 int run_backward(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src);
 int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src);

@@ -623,6 +623,7 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     const cudaError_t le = cudaGetLastError();   // launch-configuration errors are not reported by the sync
     if (le != cudaSuccess) return cuda_fail(ctx, le, "first-order step launch");
     if (fields) {
+        touch_pages({{fields, nullptr, 16 * C * 4}});   // while the time loop runs
         // the newest level: written by the last step
         const bool last_even = ((ctx->nt - 1) & 1) == 0;
         const float* v[4];
@@ -634,28 +635,20 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
         const int dst[12] = {2, 3, 4, 5, 8, 9, 10, 11, 12, 13, 14, 15};
         for (int k = 0; k < 12; k += 4) {
             launch_pack_fields(order + k, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
-            for (int q = 0; q < 4; ++q)
-                if (cudaMemcpyAsync(fields + (size_t)dst[k + q] * C, ctx->staging + (size_t)q * C, C * 4,
-                                    cudaMemcpyDeviceToHost, ctx->stream) != cudaSuccess)
-                    return fail(ctx, OUC_ECUDA, "field download failed");
-            if (cudaStreamSynchronize(ctx->stream) != cudaSuccess) return fail(ctx, OUC_ECUDA, "field download failed");
+            if ((rc = to_host(ctx, fields + (size_t)dst[k] * C, ctx->staging, 4 * C * 4))) return rc;   // 4 fields in a row
         }
+        // totals as the kernels form them: U = P + S, theta = theta_x +
+        // theta_z + s, omega = omega_x + omega_z (the source term below)
+        const float* f[4] = {v[0], v[1], st[0], st[2]};
+        const float* g[4] = {v[2], v[3], st[1], st[3]};
+        launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream, g);
+        if ((rc = to_host(ctx, fields, ctx->staging, 2 * C * 4))) return rc;
+        if ((rc = to_host(ctx, fields + 6 * C, ctx->staging + 2 * C, 2 * C * 4))) return rc;
     }
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "first-order time loop");
     if ((rc = check_status(ctx))) return rc;
-    if (fields) {
-        // totals as the kernels form them: U = P + S, theta = theta_x + theta_z + s,
-        // omega = omega_x + omega_z
-        const size_t src_cell = (size_t)(shot->sx + ctx->L) * ctx->Z + (shot->sz + ctx->L);
-        for (size_t k = 0; k < C; ++k) {
-            const float sv = k == src_cell ? theta_src : 0.0f;
-            fields[k] = fields[2 * C + k] + fields[4 * C + k];
-            fields[C + k] = fields[3 * C + k] + fields[5 * C + k];
-            fields[6 * C + k] = fields[12 * C + k] + fields[13 * C + k] + sv;
-            fields[7 * C + k] = fields[14 * C + k] + fields[15 * C + k];
-        }
-    }
+    if (fields) fields[6 * C + (size_t)(shot->sx + ctx->L) * ctx->Z + (shot->sz + ctx->L)] += theta_src;
     (backward ? ctx->timing.backward_ms : ctx->timing.forward_ms) = elapsed(ctx->ev[1], ctx->ev[2]);
     return OUC_OK;
 }
@@ -689,8 +682,7 @@ int ouc_backward_fo(ouc_ctx* ctx, const ouc_shot* shot, const float* rec_vx, con
     cudaSetDevice(ctx->device);
     ctx->step_phase = ouc_ctx::kIdle;
     ctx->timing = ouc_timing{};
-    if ((rc = gather_in(ctx, rec_vx, ctx->gather(0, 0), true))) return rc;
-    if ((rc = gather_in(ctx, rec_vz, ctx->gather(0, 1), true))) return rc;
+    if ((rc = records_in(ctx, {{rec_vx, ctx->gather(0, 0), ctx->X}, {rec_vz, ctx->gather(0, 1), ctx->X}}, true))) return rc;
     return fo_run(ctx, shot, true, 0.0f, fields);
 }
 

@@ -730,18 +730,24 @@ void launch_grad_stack(const GradStackArgs& a, cudaStream_t s) {
 
 struct PackArgs {
     const float* f[12];
+    const float* g[12];      // second addend of a sum, or null
     int nf, X, Z, pitch;
     float* out;
 };
 __global__ void k_pack(const PackArgs a) {
     const int i = blockIdx.y, k = blockIdx.z;
-    for (int j = threadIdx.x + blockIdx.x * blockDim.x; j < a.Z; j += blockDim.x * gridDim.x)
-        a.out[((size_t)k * a.X + i) * a.Z + j] = a.f[k][(ptrdiff_t)i * a.pitch + j];
+    for (int j = threadIdx.x + blockIdx.x * blockDim.x; j < a.Z; j += blockDim.x * gridDim.x) {
+        const ptrdiff_t c = (ptrdiff_t)i * a.pitch + j;
+        float v = a.f[k][c];
+        if (a.g[k]) v += a.g[k][c];
+        a.out[((size_t)k * a.X + i) * a.Z + j] = v;
+    }
 }
 
-void launch_pack_fields(const float* const* f, int nf, int X, int Z, int pitch, float* out, cudaStream_t s) {
+void launch_pack_fields(const float* const* f, int nf, int X, int Z, int pitch, float* out, cudaStream_t s,
+                        const float* const* g) {
     PackArgs a;
-    for (int k = 0; k < nf && k < 12; ++k) a.f[k] = f[k];
+    for (int k = 0; k < 12; ++k) { a.f[k] = k < nf ? f[k] : nullptr; a.g[k] = g && k < nf ? g[k] : nullptr; }
     a.nf = nf; a.X = X; a.Z = Z; a.pitch = pitch; a.out = out;
     dim3 grid((Z + 255) / 256, X, nf);
     k_pack<<<grid, 256, 0, s>>>(a);

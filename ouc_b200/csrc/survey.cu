@@ -151,20 +151,7 @@ int upload_batch(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture*
     return OUC_OK;
 }
 
-// Gathers between the caller's layout (X_b x nt or nt x X_b, host) and the
-// time-major device gather of width X_b.
-int gather_to_device(ouc_ctx* ctx, const float* src, float* dst_tx, int Xb) {
-    const size_t n = (size_t)ctx->nt * Xb;
-    if (ctx->cfg.gather_layout == OUC_GATHER_TX) {
-        CKS(cudaMemcpyAsync(dst_tx, src, n * 4, cudaMemcpyHostToDevice, ctx->stream));
-        return OUC_OK;
-    }
-    CKS(cudaMemcpyAsync(ctx->staging, src, n * 4, cudaMemcpyHostToDevice, ctx->stream));
-    launch_transpose(ctx->staging, dst_tx, Xb, ctx->nt, ctx->stream);
-    ctx->timing.kernel_launches += 1;
-    return OUC_OK;
-}
-
+// A time-major device gather of width X_b into the caller's layout (host).
 int gather_to_host(ouc_ctx* ctx, const float* src_tx, float* dst, int Xb) {
     const size_t n = (size_t)ctx->nt * Xb;
     const float* from = src_tx;
@@ -173,8 +160,7 @@ int gather_to_host(ouc_ctx* ctx, const float* src_tx, float* dst, int Xb) {
         ctx->timing.kernel_launches += 1;
         from = ctx->staging;
     }
-    CKS(cudaMemcpyAsync(dst, from, n * 4, cudaMemcpyDeviceToHost, ctx->stream));
-    return OUC_OK;
+    return to_host(ctx, dst, from, n * 4);
 }
 
 int group(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, const float* d_w, bool forward_only,
@@ -184,6 +170,7 @@ int group(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, co
     if (rc) return rc;
     const bool self_records = !forward_only && rx == nullptr;
     CKS(cudaEventRecord(ctx->ev[0], ctx->stream));
+    if (!forward_only && !self_records && (rc = records_fence(ctx))) return rc;
     if ((rc = run_forward(ctx, n, forward_only || self_records, !forward_only))) return rc;
     if (forward_only) {
         CKS(cudaEventRecord(ctx->ev[1], ctx->stream));
@@ -197,13 +184,14 @@ int group(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, co
         ctx->timing.forward_ms += elapsed(ctx->ev[0], ctx->ev[1]);
         return OUC_OK;
     }
+    std::vector<Record> recs;
     for (int b = 0; b < n && !self_records; ++b) {
         if (!rx[b] || !rz[b]) return fail(ctx, OUC_EINVAL, "record pointer missing for a shot");
         const int Xb = ap[b].x1 - ap[b].x0 + 2 * ctx->L;
-        if ((rc = gather_to_device(ctx, rx[b], ctx->gather(b, 0), Xb))) return rc;
-        if ((rc = gather_to_device(ctx, rz[b], ctx->gather(b, 1), Xb))) return rc;
-        CKS(cudaStreamSynchronize(ctx->stream));   // staging reused
+        recs.push_back({rx[b], ctx->gather(b, 0), Xb});
+        recs.push_back({rz[b], ctx->gather(b, 1), Xb});
     }
+    if ((rc = records_beside(ctx, recs, true))) return rc;
     for (int b = 0; b < n; ++b) {
         if (!shots[b].mute) continue;
         const int L = ctx->L, Xb = ap[b].x1 - ap[b].x0 + 2 * L;
@@ -244,11 +232,13 @@ int group(ouc_ctx* ctx, int n, const ouc_shot* shots, const ouc_aperture* ap, co
         launch_finalize(f, ctx->stream);
         ctx->timing.kernel_launches += 1;
     }
+    std::vector<HostCopy> images;
     for (int b = 0; b < n; ++b) {
         const size_t nib = (size_t)(ap[b].x1 - ap[b].x0) * ctx->nz;
-        if (ipp && ipp[b]) CKS(cudaMemcpyAsync(ipp[b], ctx->d_img + (size_t)(2 * b) * ni, nib * 4, cudaMemcpyDeviceToHost, ctx->stream));
-        if (ips && ips[b]) CKS(cudaMemcpyAsync(ips[b], ctx->d_img + (size_t)(2 * b) * ni + nib, nib * 4, cudaMemcpyDeviceToHost, ctx->stream));
+        if (ipp && ipp[b]) images.push_back({ipp[b], ctx->d_img + (size_t)(2 * b) * ni, nib * 4});
+        if (ips && ips[b]) images.push_back({ips[b], ctx->d_img + (size_t)(2 * b) * ni + nib, nib * 4});
     }
+    if ((rc = copy_host(ctx, images, true))) return rc;
     CKS(cudaEventRecord(ctx->ev[3], ctx->stream));
     CKS(cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
