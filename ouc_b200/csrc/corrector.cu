@@ -1,25 +1,26 @@
 // Learned dispersion corrector (include/ouc_corrector.h): a 4-layer 5x5 CNN
 // whose convolutions run as implicit GEMMs on the sm_100a tensor cores.
 //
-// A convolution's GEMM M is 128 consecutive pixels of one image row, N all
-// output channels (32 or 16), K 25 taps x input channels.  A work item is RB
-// consecutive rows of 128 pixels; its (RB + 4)-row x 132-column input patch
-// (zeros outside the image) lies in shared memory in the no-swizzle K-major "core matrix" layout -- [row][channel chunk of 8]
+// A convolution's GEMM M is 128 consecutive pixels of one image row, N the
+// output channels (32 or 16) of up to four rows, K 25 taps x input channels.
+// A work item is kCB consecutive rows of 128 pixels; its (kCB + 4)-row x
+// 132-column input patch (zeros outside the image) lies in shared memory in
+// the no-swizzle K-major "core matrix" layout -- [row][channel chunk of 8]
 // [column][8 channels], 16 bytes per (column, chunk) -- so that the A operand
 // of tap (dx, dz) is simply the patch shifted by (dx, dz): a shared-memory
 // matrix descriptor whose start address moves by 16 * (dx * chunks * 132 + dz)
 // bytes, with the leading-dimension offset = one chunk plane (132 * 16 B)
 // and the stride offset = 8 pixels (128 B).  No im2col copy is made.  The
 // weights of all taps sit in shared memory for the whole (persistent) CTA in
-// the same layout, [tap][chunk][out channel][8].  The roles are split over
-// warps and the items pipelined two deep: eight warps copy (16-byte
-// asynchronous copies; tensor copies of this layout, whose innermost extent
-// is 16 bytes, were no faster), one thread issues the 25 * (channels / 16) tcgen05.mma instructions per row (kind::f16,
-// BF16 x BF16 -> FP32 in tensor memory), and four warps read the finished
-// 128 x N accumulators back with tcgen05.ld (warp w owns lanes 32w..32w+31,
-// i.e. pixels 32w..32w+31) for the epilogue: bias + ReLU -> BF16 activations,
-// bias -> FP32 outputs, or (input-gradient pass) the ReLU mask of the forward
-// activation.
+// the same kind of layout, [dz][chunk][dx, descending][out channel][8].  The
+// roles are split over warps and the items pipelined two deep: eight warps
+// copy (16-byte asynchronous copies; tensor copies of this layout, whose
+// innermost extent is 16 bytes, were no faster), one thread issues the
+// tcgen05.mma instructions (kind::f16, BF16 x BF16 -> FP32 in tensor memory),
+// and four warps read the finished 128 x N accumulators back with tcgen05.ld
+// (warp w owns lanes 32w..32w+31, i.e. pixels 32w..32w+31) for the epilogue:
+// bias + ReLU -> BF16 activations, bias -> FP32 outputs, or (input-gradient
+// pass) the ReLU mask of the forward activation.
 //
 // Every wait is bounded: an mbarrier that does not complete within ~2 s
 // sets the network's error flag; the CTA then waits once more (also
@@ -47,7 +48,8 @@ constexpr int kTile = 128;            // GEMM M: pixels per tile
 constexpr int kPC = kTile + 4;        // patch columns (2 + 2 halo)
 constexpr int kTaps = 25;
 constexpr int kMaxPairs = 32 * 32;     // (cin, cout) pairs of the widest layer
-constexpr int kRB = 2;                 // image rows of a work item
+constexpr int kRB = 2;                 // image rows of a weight-gradient work item
+constexpr int kCB = 4;                 // image rows of a convolution work item
 constexpr int kWgradCtas = 148;        // CTAs (partial-sum slots) of k_wgrad_tc
 constexpr int kBgradBlocks = 592;      // blocks of k_bgrad
 constexpr int kCopyThreads = 256;      // copy warps 5-12
@@ -195,15 +197,16 @@ struct ConvArgs {
     int* err;
 };
 
-// Work items of kRB rows x 128 pixels.
+// Work items of RB rows x 128 pixels.
+template <int RB>
 struct Items {
     int tiles_w, row_blocks, count;
     __host__ __device__ Items(int n, int H, int W)
-        : tiles_w((W + kTile - 1) / kTile), row_blocks((H + kRB - 1) / kRB), count(n * row_blocks * tiles_w) {}
+        : tiles_w((W + kTile - 1) / kTile), row_blocks((H + RB - 1) / RB), count(n * row_blocks * tiles_w) {}
     __device__ __forceinline__ void at(int item, int& img, int& h, int& z0) const {
         const int tw = item % tiles_w, rest = item / tiles_w;
         img = rest / row_blocks;
-        h = (rest - img * row_blocks) * kRB;
+        h = (rest - img * row_blocks) * RB;
         z0 = tw * kTile;
     }
 };
@@ -245,18 +248,25 @@ struct ConvGeo {
     static constexpr int NQ = CIN / 8;
     static constexpr int w_bytes = kTaps * CIN * COUT * 2;
     static constexpr int row_bytes = NQ * kPC * 16;
-    static constexpr int p_bytes = (kRB + 4) * row_bytes;     // one stage
+    static constexpr int p_bytes = (kCB + 4) * row_bytes;     // one stage
     static constexpr int bytes = w_bytes + 2 * p_bytes;
-    static constexpr int acc_cols = 2 * kRB * COUT;
-    static constexpr int tmem_cols = acc_cols <= 32 ? 32 : acc_cols <= 64 ? 64 : acc_cols <= 128 ? 128 : 256;
+    static constexpr int acc_cols = 2 * kCB * COUT;
+    static constexpr int tmem_cols = acc_cols <= 128 ? 128 : 256;
     static_assert(acc_cols <= 256, "two accumulator stages fit tensor memory");
-    static_assert(w_bytes % 128 == 0 && row_bytes % 128 == 0, "tensor-copy destinations are 128-byte aligned");
 };
 
-// Bound: the MMAs, about 85 cycles each whatever their 16 or 32 columns (the
-// same with the copies left out).  A 32 -> 32 layer on 4 images of 290 x 158:
-// 72 -> 33 us (first form: 128 threads
-// staged the patch of one row, then waited for its MMAs).
+// An input row i of an item (row h - 2 + i of the image) feeds the output rows
+// o = i - dx, dx = 0 .. 4, with one A operand per column shift dz and channel
+// chunk pair.  The accumulators of the item's rows lie side by side in tensor
+// memory and the weights of the five dx side by side, in descending dx, in
+// shared memory, so one MMA serves all of them (N up to 4 x COUT): 83 MMAs per
+// item instead of 200.  Input rows run upwards, so that every output row
+// still sums its taps in the order dx, dz, channel.
+//
+// Bound: the MMAs, about 85 cycles each nearly whatever their N (the same
+// with the copies left out).  A 32 -> 32 layer on 4 images of 290 x 158:
+// 72 us at first (128 threads staged the patch of one row, then waited for its
+// MMAs), 33 us pipelined with an MMA per tap, 24 us with one for five.
 template <int CIN, int COUT, int EPI>
 __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
     using G = ConvGeo<CIN, COUT>;
@@ -267,7 +277,7 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
     __shared__ __align__(8) uint64_t full[2], done[2], drained[2];   // copied; multiplied; accumulators read
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const Items items(a.n, a.H, a.W);
+    const Items<kCB> items(a.n, a.H, a.W);
 
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
@@ -276,7 +286,11 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
             mbar_init(&drained[s], 128);
         }
     }
-    for (int i = tid; i < G::w_bytes / 16; i += kThreadsConv) cp16(smem_u32(s_w) + i * 16, a.w + i * 8, true);
+    // weights [tap = dx 5 + dz][chunk][out channel][8] -> [dz][chunk][4 - dx][out channel][8]
+    for (int i = tid; i < G::w_bytes / 16; i += kThreadsConv) {
+        const int co = i % COUT, q = i / COUT % NQ, tap = i / (COUT * NQ), dx = tap / 5, dz = tap - 5 * dx;
+        cp16(smem_u32(s_w) + (((dz * NQ + q) * 5 + 4 - dx) * COUT + co) * 16, a.w + (size_t)i * 8, true);
+    }
     cp_commit();
     cp_wait<0>();
     fence_proxy_async();
@@ -295,13 +309,12 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
             if (k >= 2 && !(ok = mbar_wait(&done[s], (uint32_t)((k >> 1) - 1) & 1u))) break;
             int img, h, z0;
             items.at(it, img, h, z0);
-            copy_patch<CIN, kRB + 4, kPC>(smem_u32(s_p) + s * G::p_bytes, a.x, img, h - 2, z0 - 2, a.H, a.W, tid - 160);
+            copy_patch<CIN, kCB + 4, kPC>(smem_u32(s_p) + s * G::p_bytes, a.x, img, h - 2, z0 - 2, a.H, a.W, tid - 160);
             cp_commit();
         }
         if (k > 0 && ok) hand_over(&full[(k - 1) & 1]);
     } else if (tid == 128) {   // MMAs
-        const uint64_t bd0 = umma_desc(smem_u32(s_w), COUT * 16, 128);
-        constexpr uint32_t idesc = idesc_bf16(kTile, COUT);
+        const uint64_t bd0 = umma_desc(smem_u32(s_w), 5 * COUT * 16, 128);
         int k = 0;
         for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
             const int s = k & 1;
@@ -312,20 +325,21 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
             // descriptors: the start address (in 16-byte units) is the low
             // field, so a tap or chunk is one addition
             const uint64_t ad0 = umma_desc(smem_u32(s_p) + s * G::p_bytes, kPC * 16, 128);
-#pragma unroll 1
-            for (int r = 0; r < kRB; ++r) {
-                const uint32_t d = tmem + (uint32_t)((s * kRB + r) * COUT);
+            const uint32_t d0 = tmem + (uint32_t)(s * kCB * COUT);
 #pragma unroll
-                for (int dx = 0; dx < 5; ++dx) {
-                    const uint64_t adr = ad0 + (uint32_t)((r + dx) * NQ * kPC);
+            for (int i = 0; i < kCB + 4; ++i) {
+                const int o0 = i > 4 ? i - 4 : 0, o1 = i < kCB ? i : kCB - 1;   // output rows o0 .. o1
+                const int b0 = 4 - (i - o0);                                    // block of dx = i - o0
 #pragma unroll
-                    for (int dz = 0; dz < 5; ++dz) {
+                for (int dz = 0; dz < 5; ++dz) {
 #pragma unroll
-                        for (int ks = 0; ks < NQ / 2; ++ks) {
-                            const int tap = dx * 5 + dz;
-                            umma_bf16(d, adr + (uint32_t)(2 * ks * kPC + dz), bd0 + (uint32_t)((tap * NQ + 2 * ks) * COUT), idesc,
-                                      tap || ks ? 1u : 0u);
-                        }
+                    for (int ks = 0; ks < NQ / 2; ++ks) {
+                        const uint64_t ad = ad0 + (uint32_t)((i * NQ + 2 * ks) * kPC + dz);
+                        const uint64_t bd = bd0 + (uint32_t)(((dz * NQ + 2 * ks) * 5 + b0) * COUT);
+                        const bool first = i < kCB && dz == 0 && ks == 0;       // row i's first product overwrites
+                        const int n = o1 - o0 + (first ? 0 : 1);
+                        if (n > 0) umma_bf16(d0 + (uint32_t)(o0 * COUT), ad, bd, idesc_bf16(kTile, n * COUT), 1u);
+                        if (first) umma_bf16(d0 + (uint32_t)(i * COUT), ad, bd + (uint32_t)((i - o0) * COUT), idesc_bf16(kTile, COUT), 0u);
                     }
                 }
             }
@@ -340,25 +354,25 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
             ok = __all_sync(0xffffffffu, mbar_wait(&done[s], (uint32_t)(k >> 1) & 1u));
             if (!ok) break;
             tc_fence_after();
-            uint32_t r[kRB][COUT];
-#pragma unroll
-            for (int q = 0; q < kRB; ++q)
-                tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((s * kRB + q) * COUT), r[q]);
-            tc_fence_before();
-            mbar_arrive(&drained[s]);
             int img, h, z0;
             items.at(it, img, h, z0);
             const int gz = z0 + warp * 32 + lane;
-            if (gz >= a.W) continue;
-#pragma unroll
-            for (int q = 0; q < kRB; ++q) {
-                if (h + q >= a.H) break;
+#pragma unroll 1
+            for (int q = 0; q < kCB; ++q) {
+                uint32_t r[COUT];
+                __syncwarp();
+                tmem_ld<COUT>(tmem + ((uint32_t)(warp * 32) << 16) + (uint32_t)((s * kCB + q) * COUT), r);
+                if (q == kCB - 1) {
+                    tc_fence_before();
+                    mbar_arrive(&drained[s]);
+                }
+                if (gz >= a.W || h + q >= a.H) continue;
                 const size_t p = ((size_t)img * a.H + h + q) * a.W + gz;
                 if (EPI == kOut) {
                     float* y = static_cast<float*>(a.y) + p * a.cout_real;
 #pragma unroll
                     for (int c = 0; c < COUT; ++c)
-                        if (c < a.cout_real) y[c] = __uint_as_float(r[q][c]) + a.bias[c];   // the caller's buffer: float-aligned
+                        if (c < a.cout_real) y[c] = __uint_as_float(r[c]) + a.bias[c];   // the caller's buffer: float-aligned
                 } else {
                     uint4* y = reinterpret_cast<uint4*>(static_cast<bf16*>(a.y) + p * COUT);
                     const uint4* mk = EPI == kDgrad ? reinterpret_cast<const uint4*>(a.mask + p * COUT) : nullptr;
@@ -370,7 +384,7 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
 #pragma unroll
                         for (int e = 0; e < 8; ++e) {
                             const int c = 8 * c8 + e;
-                            float v = __uint_as_float(r[q][c]);
+                            float v = __uint_as_float(r[c]);
                             if (EPI == kHidden) v = fmaxf(v + a.bias[c], 0.f);
                             else v = __bfloat162float(mv[e]) > 0.f ? v : 0.f;
                             o[e] = __float2bfloat16_rn(v);
@@ -399,7 +413,7 @@ cudaError_t launch_conv(const ConvArgs& a, int sms, cudaStream_t s) {
     const cudaError_t e =
         cudaFuncSetAttribute(k_conv5<CIN, COUT, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
-    const int count = Items(a.n, a.H, a.W).count;
+    const int count = Items<kCB>(a.n, a.H, a.W).count;
     k_conv5<CIN, COUT, EPI><<<count < sms ? count : sms, kThreadsConv, bytes, s>>>(a);
     return cudaSuccess;
 }
@@ -472,7 +486,7 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_wgrad_tc(int n, int H, int 
     __shared__ __align__(8) uint64_t full[2], done[2];
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const Items items(n, H, W);
+    const Items<kRB> items(n, H, W);
     const int mine = items.count > (int)blockIdx.x ? (items.count - 1 - blockIdx.x) / gridDim.x + 1 : 0;   // items of this CTA
 
     if (tid == 0)
@@ -574,7 +588,7 @@ cudaError_t launch_wgrad(int n, int H, int W, const bf16* x, const bf16* g, int 
     const cudaError_t e = cudaFuncSetAttribute(k_wgrad_tc<CIN, COUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     if (e != cudaSuccess) return e;
     // a fixed grid (at most kWgradCtas partial-sum slots), independent of the device
-    const int count = Items(n, H, W).count, grid = count < kWgradCtas ? count : kWgradCtas;
+    const int count = Items<kRB>(n, H, W).count, grid = count < kWgradCtas ? count : kWgradCtas;
     k_wgrad_tc<CIN, COUT><<<grid, kThreadsConv, bytes, s>>>(n, H, W, x, g, cin_real, cout_real, part, err);
     *nblocks = grid;
     return cudaSuccess;
@@ -615,31 +629,33 @@ __global__ void __launch_bounds__(256) k_bgrad(size_t npix, const bf16* g, float
     }
 }
 
-// dw[co][ci][tap] += the CTAs' partial sums in a fixed order: four threads
-// each add a quarter of the CTAs in order, then the four; the last block
-// adds the bias sums, a warp per channel, lanes striding the blocks and a
+// dw[co][ci][tap] += the CTAs' partial sums in a fixed order: eight threads
+// each add an eighth of the CTAs in order, then the eight; the last four blocks
+// add the bias sums, a warp per channel, lanes striding the blocks and a
 // fixed tree over the lanes.
 __global__ void __launch_bounds__(256) k_grad_sum(int nblocks, int cin_real, int cout_real, const float* part, float* dw,
                                                   int nbias, const float* bpart, float* db) {
-    if (blockIdx.x == gridDim.x - 1) {
-        const int lane = threadIdx.x & 31;
-        for (int c = threadIdx.x >> 5; c < cout_real; c += 8) {
-            float s = 0.f;
-#pragma unroll 4
-            for (int b = lane; b < nbias; b += 32) s += bpart[(size_t)b * 32 + c];
+    if (blockIdx.x >= gridDim.x - 4) {
+        const int lane = threadIdx.x & 31, c = 8 * (int)(blockIdx.x - (gridDim.x - 4)) + (threadIdx.x >> 5);
+        if (c >= cout_real) return;
+        float s = 0.f;
 #pragma unroll
-            for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-            if (lane == 0) db[c] += s;
+        for (int k = 0; k < (kBgradBlocks + 31) / 32; ++k) {
+            const int b = lane + 32 * k;
+            if (b < nbias) s += bpart[(size_t)b * 32 + c];
         }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+        if (lane == 0) db[c] += s;
         return;
     }
-    __shared__ float red[4][64];
-    const int npairs = cin_real * cout_real, grp = threadIdx.x >> 6, t = threadIdx.x & 63;
-    const int i = blockIdx.x * 64 + t;
+    __shared__ float red[8][32];
+    const int npairs = cin_real * cout_real, grp = threadIdx.x >> 5, t = threadIdx.x & 31;
+    const int i = blockIdx.x * 32 + t;
     const bool in = i < kTaps * npairs;
     const int tap = in ? i / npairs : 0, pr = in ? i - tap * npairs : 0;
     const float* p = part + (size_t)tap * kMaxPairs + pr;
-    const int b0 = nblocks * grp / 4, b1 = nblocks * (grp + 1) / 4;
+    const int b0 = nblocks * grp / 8, b1 = nblocks * (grp + 1) / 8;
     float s = 0.f;
 #pragma unroll 8
     for (int b = b0; b < b1; ++b) s += p[(size_t)b * kTaps * kMaxPairs];
@@ -647,7 +663,10 @@ __global__ void __launch_bounds__(256) k_grad_sum(int nblocks, int cin_real, int
     __syncthreads();
     if (grp == 0 && in) {
         const int ci = pr % cin_real, co = pr / cin_real;
-        dw[((size_t)co * cin_real + ci) * kTaps + tap] += ((red[0][t] + red[1][t]) + red[2][t]) + red[3][t];
+        float v = red[0][t];
+#pragma unroll
+        for (int k = 1; k < 8; ++k) v += red[k][t];
+        dw[((size_t)co * cin_real + ci) * kTaps + tap] += v;
     }
 }
 
@@ -890,7 +909,7 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
         cudaSuccess)
         return OUC_ECUDA;
     k_bgrad<16><<<kBgradBlocks, 256, 0, s>>>(P, net->g16, net->bpart);
-    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[3].cin, kL[3].cout, net->part, gp + p_offset(3), kBgradBlocks, net->bpart,
+    k_grad_sum<<<kTaps * kMaxPairs / 32 + 4, 256, 0, s>>>(nb, kL[3].cin, kL[3].cout, net->part, gp + p_offset(3), kBgradBlocks, net->bpart,
                                    gp + p_offset(3) + w_count(3));
     ConvArgs a{};
     a.n = n; a.H = H; a.W = W; a.err = net->err;
@@ -903,7 +922,7 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
             cudaSuccess)
             return OUC_ECUDA;
         k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, gl, net->bpart);
-    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l), kBgradBlocks, net->bpart,
+    k_grad_sum<<<kTaps * kMaxPairs / 32 + 4, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l), kBgradBlocks, net->bpart,
                                    gp + p_offset(l) + w_count(l));
         a.x = gl; a.w = net->wd[l]; a.mask = net->y[l - 1]; a.y = net->g[(3 - l) & 1];
         if (launch_conv<32, 32, kDgrad>(a, net->sms, s) != cudaSuccess) return OUC_ECUDA;
@@ -913,7 +932,7 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
     if (launch_wgrad<16, 32>(n, H, W, net->x0, g1, kL[0].cin, kL[0].cout, net->part, net->err, &nb, s) != cudaSuccess)
         return OUC_ECUDA;
     k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, g1, net->bpart);
-    k_grad_sum<<<kTaps * kMaxPairs / 64 + 1, 256, 0, s>>>(nb, kL[0].cin, kL[0].cout, net->part, gp + p_offset(0), kBgradBlocks, net->bpart,
+    k_grad_sum<<<kTaps * kMaxPairs / 32 + 4, 256, 0, s>>>(nb, kL[0].cin, kL[0].cout, net->part, gp + p_offset(0), kBgradBlocks, net->bpart,
                                    gp + p_offset(0) + w_count(0));
     return cudaGetLastError() == cudaSuccess ? OUC_OK : OUC_ECUDA;
 }

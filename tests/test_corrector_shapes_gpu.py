@@ -1,5 +1,5 @@
-"""Edges of the corrector convolutions' work items (2 image rows x 128
-pixels): images of one row, odd heights, widths one below, at and one above
+"""Edges of the corrector convolutions' work items (4 image rows x 128
+pixels, 2 rows for the weight gradients): images of one row, odd heights, widths one below, at and one above
 128 and 256, the narrowest images, and more items than CTAs, against the CPU
 restatement oracle/cnn.py with the tolerances of test_corrector_gpu.py (the
 same operand roundings; FP32 accumulation in another order may move an
