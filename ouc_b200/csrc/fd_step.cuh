@@ -166,17 +166,36 @@ __device__ __forceinline__ float div_tiny(float x, float h, float r) {
     }
     return copysignf(q, x);
 }
-__device__ __forceinline__ float4 div4(float4 x, const Div& d) {
+__device__ __forceinline__ float4 div4_fast(float4 x, const Div& d) {
     const float2 q0l = mul2(lo2(x), dup2(d.r)), q0h = mul2(hi2(x), dup2(d.r));
-    float4 q = cat4(fma2(fma2(q0l, dup2(-d.h), lo2(x)), dup2(d.r), q0l),
-                    fma2(fma2(q0h, dup2(-d.h), hi2(x)), dup2(d.r), q0h));
-    // 0 < |x| < T, on the bits: 2 bits(x) - 1 drops the sign and wraps a zero to the largest value
-    const bool tiny = (__float_as_uint(x.x) * 2u - 1u < d.tb) | (__float_as_uint(x.y) * 2u - 1u < d.tb) |
-                      (__float_as_uint(x.z) * 2u - 1u < d.tb) | (__float_as_uint(x.w) * 2u - 1u < d.tb);
-    if (tiny)
-        q = make_float4(div_tiny(x.x, d.h, d.r), div_tiny(x.y, d.h, d.r), div_tiny(x.z, d.h, d.r),
-                        div_tiny(x.w, d.h, d.r));
+    return cat4(fma2(fma2(q0l, dup2(-d.h), lo2(x)), dup2(d.r), q0l), fma2(fma2(q0h, dup2(-d.h), hi2(x)), dup2(d.r), q0h));
+}
+// 0 < |x| < T for any of the four, on the bits: 2 bits(x) - 1 drops the sign
+// and wraps a zero to the largest value
+__device__ __forceinline__ bool any_tiny(float4 x, const Div& d) {
+    return (__float_as_uint(x.x) * 2u - 1u < d.tb) | (__float_as_uint(x.y) * 2u - 1u < d.tb) |
+           (__float_as_uint(x.z) * 2u - 1u < d.tb) | (__float_as_uint(x.w) * 2u - 1u < d.tb);
+}
+__device__ __forceinline__ float4 div4_tiny(float4 x, const Div& d) {
+    return make_float4(div_tiny(x.x, d.h, d.r), div_tiny(x.y, d.h, d.r), div_tiny(x.z, d.h, d.r), div_tiny(x.w, d.h, d.r));
+}
+__device__ __forceinline__ float4 div4(float4 x, const Div& d) {
+    float4 q = div4_fast(x, d);
+    if (any_tiny(x, d)) q = div4_tiny(x, d);
     return q;
+}
+// Two quads with one branch between them (16 shots of 1060 x 560, against a
+// branch per quad: forward 274 -> 261 us, receiver 230 -> 222, reconstruction
+// 249 -> 243; four quads per branch were no better).
+__device__ __forceinline__ void div4_pair(float4& x, float4& y, const Div& d) {
+    const bool tx = any_tiny(x, d), ty = any_tiny(y, d);
+    float4 qx = div4_fast(x, d), qy = div4_fast(y, d);
+    if (tx | ty) {
+        if (tx) qx = div4_tiny(x, d);
+        if (ty) qy = div4_tiny(y, d);
+    }
+    x = qx;
+    y = qy;
 }
 // CPML memory update fma(fma(d, e, -(d m)), dt, m), packed
 __device__ __forceinline__ float2 cpml2(float2 m, float2 d, float2 e, float dt) {
@@ -192,7 +211,7 @@ __device__ __forceinline__ float4 cpml4(float4 m, float4 d, float4 e, float dt) 
 // PLUS: sum_k a_k (f[j+k] - f[j-k+1]);  MINUS: sum_k a_k (f[j+k-1] - f[j-k]).
 // Scalar: the z-shifted pairs do not sit in aligned register pairs.
 template <int N, bool PLUS>
-__device__ __forceinline__ float4 dz4(const float* row, const float* a, const Div& dv) {
+__device__ __forceinline__ float4 dz4_sum(const float* row, const float* a) {
     constexpr int NB = (N + 3) / 4;
     float w[4 * (2 * NB + 1)];
 #pragma unroll
@@ -214,7 +233,11 @@ __device__ __forceinline__ float4 dz4(const float* row, const float* a, const Di
                        : __fmaf_rn(a[k], __fsub_rn(w[c + k], w[c - k - 1]), acc);
         o[q] = acc;
     }
-    return div4(make_float4(o[0], o[1], o[2], o[3]), dv);
+    return make_float4(o[0], o[1], o[2], o[3]);
+}
+template <int N, bool PLUS>
+__device__ __forceinline__ float4 dz4(const float* row, const float* a, const Div& dv) {
+    return div4(dz4_sum<N, PLUS>(row, a), dv);
 }
 
 // Staggered x derivatives of RR consecutive rows of one float4 column,
@@ -244,7 +267,13 @@ __device__ __forceinline__ void dx4(const float* col, int st, const float* a, co
             acl = fma2(dup2(a[k]), sub2(lo2(w[hi]), lo2(w[lo])), acl);
             ach = fma2(dup2(a[k]), sub2(hi2(w[hi]), hi2(w[lo])), ach);
         }
-        out[q] = div4(cat4(acl, ach), dv);
+        out[q] = cat4(acl, ach);
+    }
+    if constexpr (RR == 2) {
+        div4_pair(out[0], out[1], dv);
+    } else {
+#pragma unroll
+        for (int q = 0; q < RR; ++q) out[q] = div4(out[q], dv);
     }
 }
 
@@ -795,8 +824,9 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
             const int r = r0 + q;
             const int gi = x0 + r;
             const int gjb = z0 + c;
-            const float4 exz = dz4<N, true>(ux0 + q * UC, a, dvz);    // dvxdz = D+z Ux
-            const float4 ezz = dz4<N, false>(uz0 + q * UC, a, dvz);   // dvzdz = D-z Uz
+            float4 exz = dz4_sum<N, true>(ux0 + q * UC, a);    // dvxdz = D+z Ux
+            float4 ezz = dz4_sum<N, false>(uz0 + q * UC, a);   // dvzdz = D-z Uz
+            div4_pair(exz, ezz, dvz);
             const int g = gi * P + gjb;
             const float4 vp2 = vp2r[qq], vs2 = vs2r[qq];
             const bool own = ownc && r >= 0 && r < TX;
@@ -994,10 +1024,12 @@ __device__ __forceinline__ bool step_tile(const StepArgs& p, const Geo& gm, cons
                 dx4<N, 1, false>(sQxz + (r + SHX) * TZ + c, TZ, a, dvx, dB);     // dux_zdx = D-x Qxz
                 dx4<N, 1, true>(sQzz + (r + SHX) * TZ + c, TZ, a, dvx, dE);      // duz_zdx = D+x Qzz
             }
-            const float4 tz = dz4<N, true>(sTh + (r + SHX) * SC + scol, a, dvz);    // dthetadz
-            const float4 wz = dz4<N, false>(sOm + (r + SHX) * SC + scol, a, dvz);   // domegadz
-            const float4 dA = dz4<N, true>(sQxx + r * SC + scol, a, dvz);           // dux_xdz = D+z Qxx
-            const float4 dC = dz4<N, false>(sQzx + r * SC + scol, a, dvz);          // duz_xdz = D-z Qzx
+            float4 tz = dz4_sum<N, true>(sTh + (r + SHX) * SC + scol, a);    // dthetadz
+            float4 wz = dz4_sum<N, false>(sOm + (r + SHX) * SC + scol, a);   // domegadz
+            div4_pair(tz, wz, dvz);
+            float4 dA = dz4_sum<N, true>(sQxx + r * SC + scol, a);           // dux_xdz = D+z Qxx
+            float4 dC = dz4_sum<N, false>(sQzx + r * SC + scol, a);          // duz_xdz = D-z Qzx
+            div4_pair(dA, dC, dvz);
             float4 oC = zero4(), oE = zero4(), oB = zero4(), oA = zero4();
             float4 oTx = zero4(), oTz = zero4(), oWz = zero4(), oWx = zero4();
             if (f.pz) {
