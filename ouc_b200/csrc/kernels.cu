@@ -88,8 +88,10 @@ static bool fits24(Mode mode, const StepArgs& a, int N) {
 //     1060 x 560, 2 shots 95.7         87.7        71.7       43.0    46.5
 //     1060 x 560, 4 shots  -            -            -        84.5    82.3
 // Small tiles in one wave: one CTA of 576 threads per SM (16 rows) or of 768
-// (24 rows); two of 576 with fewer registers each up to two per SM.  Beyond
-// that 16 x 64 tiles, whose last wave is half as long as a 32 x 64 one, until
+// (24 rows); two of 576 with fewer registers each up to two per SM and a
+// third of a wave more (306 tiles, half-order 2: 10.9 against 11.9 us on 16 x
+// 64 tiles; 334, a back-step of 296 x 296: 15.4 against 18.3; 350: 17.4
+// against 14.9).  Beyond that 16 x 64 tiles, whose last wave is half as long as a 32 x 64 one, until
 // the launch has about five waves of them; then the 32 x 64 tiles, which
 // recompute less halo.
 Tier pick_tier(int N, const StepArgs* rec, const StepArgs* other, Mode other_mode, int nshots) {
@@ -106,7 +108,7 @@ Tier pick_tier(int N, const StepArgs* rec, const StepArgs* other, Mode other_mod
     const int set = (other ? other : rec)->nsm, nsm = set > 0 ? set : 148;
     if (t16 <= nsm) return kSmall16;
     if (t24 <= nsm && ok24) return kSmall24;
-    if (t16 <= 2 * nsm) return kSmall16x2;
+    if (t16 <= 2 * nsm + nsm / 3) return kSmall16x2;
     return mid <= 10 * nsm ? kMid : kLarge;
 }
 
