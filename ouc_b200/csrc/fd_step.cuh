@@ -327,19 +327,27 @@ __device__ __forceinline__ void tma_prefetch_box4(const CUtensorMap* map, int c0
                  "r"(c0), "r"(c1), "r"(c2), "r"(c3)
                  : "memory");
 }
-// Programmatic dependent launch.  The step kernels are launched so that a
-// launch may start while the one before it in the stream still runs
-// (launch_pdl): they read launch constants (arguments, shot descriptors,
-// models, strips of earlier phases) first, let their own successor start at
-// once, and touch the wavefields only after pdl_wait, which returns when the
-// previous launch has completed and its writes are visible (at once when the
-// launch was an ordinary one).
+// Programmatic dependent launch.  A step launch may start while the launch
+// before it in the stream still runs (launch_pdl): its CTAs read launch
+// constants (arguments, shot descriptors, models) first and touch wavefields,
+// gathers and strips only after pdl_wait, which returns when the launch before
+// has completed and its writes are visible (at once when this launch was an
+// ordinary one).  What is read ahead of pdl_wait must therefore not be written
+// by the kernel directly ahead in the stream: a kernel that never triggers
+// does so when its blocks exit, and then only pdl_wait makes its writes
+// visible.  The first step behind a kernel that writes descriptors or models
+// is an ordinary launch (StepArgs::ordinary), unless a copy or a memset lies
+// between the two.  The small tiles, the first-order tiles and the tiles outside
+// the update domain also let their successor start at once
+// (pdl_launch_dependents); working 32 x 64 and 16 x 64 tiles do not, so behind
+// such a launch only the tail of its last CTAs overlaps.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // Launch with programmatic stream serialization: the kernel may start before
 // the launch ahead of it in the stream has finished (pdl_wait orders them).
+// ordinary: without it.
 template <class... P, class... A>
-inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, const A&... args) {
+inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, cudaStream_t s, bool ordinary, const A&... args) {
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -349,7 +357,7 @@ inline void launch_pdl(void (*kernel)(P...), dim3 grid, int threads, int smem, c
     c.dynamicSmemBytes = smem;
     c.stream = s;
     c.attrs = at;
-    c.numAttrs = 1;
+    c.numAttrs = ordinary ? 0 : 1;
     cudaLaunchKernelEx(&c, kernel, args...);
 }
 __device__ __forceinline__ void fence_proxy_async() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }

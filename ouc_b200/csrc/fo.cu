@@ -524,11 +524,11 @@ void launch(FoArgs& a, Tier tier, cudaStream_t s) {
     const int tx = tier == kLarge ? 32 : tier == kSmall24 ? 24 : 16, tz = tier == kLarge || tier == kMid ? 64 : 32;
     a.tiles_z = (a.Z + tz - 1) / tz;
     const dim3 grid((a.X + tx - 1) / tx * a.tiles_z);
-    if (tier == kLarge) launch_pdl(k_fo<N, TileGeo<N>>, grid, kThreads, TileGeo<N>::bytes, s, a);
-    else if (tier == kMid) launch_pdl(k_fo<N, MidGeo<N>>, grid, kThreads, MidGeo<N>::bytes, s, a);
-    else if (tier == kSmall24) launch_pdl(k_fo_small<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, a);
-    else if (tier == kSmall16) launch_pdl(k_fo_small<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a);
-    else launch_pdl(k_fo_small<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a);
+    if (tier == kLarge) launch_pdl(k_fo<N, TileGeo<N>>, grid, kThreads, TileGeo<N>::bytes, s, false, a);
+    else if (tier == kMid) launch_pdl(k_fo<N, MidGeo<N>>, grid, kThreads, MidGeo<N>::bytes, s, false, a);
+    else if (tier == kSmall24) launch_pdl(k_fo_small<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, false, a);
+    else if (tier == kSmall16) launch_pdl(k_fo_small<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, false, a);
+    else launch_pdl(k_fo_small<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, false, a);
 }
 
 // Five-digit weights of the reference's first-order kernels (PS:405,

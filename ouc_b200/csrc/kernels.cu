@@ -128,21 +128,21 @@ static void launch_one(const StepArgs& a, int tiles_x, int nshots, cudaStream_t 
     const Mode mode = (Mode)MODE;
     const Tier tier = a.tier != kAuto ? (Tier)a.tier : pick_tier(N, nullptr, &a, mode, nshots);
     if (tier == kLarge) {
-        launch_pdl(k_step<N, MODE>, dim3(tiles_x * a.tiles_z, nshots), kThreads, TileGeo<N>::bytes, s, a);
+        launch_pdl(k_step<N, MODE>, dim3(tiles_x * a.tiles_z, nshots), kThreads, TileGeo<N>::bytes, s, a.ordinary, a);
         return;
     }
     StepArgs b = a;
     if (tier == kMid) {
         const Grid g = grid_of(mode, a, 16, 64);
-        launch_pdl(k_step<N, MODE, MidGeo<N>>, dim3(g.tiles, nshots), kThreads, MidGeo<N>::bytes, s, b);
+        launch_pdl(k_step<N, MODE, MidGeo<N>>, dim3(g.tiles, nshots), kThreads, MidGeo<N>::bytes, s, a.ordinary, b);
         return;
     }
     const Grid g = grid_of(mode, a, tier == kSmall24 ? 24 : 16, 32);
     const dim3 grid(g.tiles, nshots);
     b.tiles_z = g.tiles_z;
-    if (tier == kSmall24) launch_pdl(k_small<N, MODE, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, b);
-    else if (tier == kSmall16) launch_pdl(k_small<N, MODE, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, b);
-    else launch_pdl(k_small<N, MODE, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, b);
+    if (tier == kSmall24) launch_pdl(k_small<N, MODE, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, a.ordinary, b);
+    else if (tier == kSmall16) launch_pdl(k_small<N, MODE, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a.ordinary, b);
+    else launch_pdl(k_small<N, MODE, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a.ordinary, b);
 }
 
 template <int N>
@@ -153,9 +153,9 @@ static int launch_back_n(const StepArgs& rec, const StepArgs& rcv, Tier tier, in
     a0.tiles_z = g0.tiles_z;
     a1.tiles_z = g1.tiles_z;
     const dim3 grid(g0.tiles + g1.tiles, nshots);
-    if (tier == kSmall24) launch_pdl(k_small_back<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, a0, a1, g0.tiles);
-    else if (tier == kSmall16) launch_pdl(k_small_back<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a0, a1, g0.tiles);
-    else if (tier == kSmall16x2) launch_pdl(k_small_back<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, a0, a1, g0.tiles);
+    if (tier == kSmall24) launch_pdl(k_small_back<N, 24, 1>, grid, SmallGeo<N, 24>::NT, SmallGeo<N, 24>::bytes, s, rec.ordinary, a0, a1, g0.tiles);
+    else if (tier == kSmall16) launch_pdl(k_small_back<N, 16, 1>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, rec.ordinary, a0, a1, g0.tiles);
+    else if (tier == kSmall16x2) launch_pdl(k_small_back<N, 16, 2>, grid, SmallGeo<N, 16>::NT, SmallGeo<N, 16>::bytes, s, rec.ordinary, a0, a1, g0.tiles);
     else return 1;
     return 0;
 }

@@ -222,6 +222,7 @@ extern "C" int ouc_forward_noalloc(const ouc_config* cfg, const ouc_shot* shot, 
         }
         for (int q = 0; q < 8; ++q) a.o[q] = o[q];
         a.t = t;
+        a.ordinary = t == 0;   // k_put_desc, directly ahead, writes the descriptor that a step reads first
         if (launch_step(N, kFwd, a, tiles_x, 1, stream)) return OUC_EINVAL;
         for (int q = 0; q < 4; ++q) {
             float* tmp = now[q]; now[q] = past[q]; past[q] = tmp;

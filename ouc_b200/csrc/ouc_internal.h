@@ -181,6 +181,7 @@ struct StepArgs {
     int comp_image;                   // kRec: compensated (Kahan) imaging sums, comp[] below
     int density;                      // variable density: scale the U-stage by the buoyancy
     int tier;                         // Tier of the launch; kAuto: chosen for it alone
+    int ordinary;                     // launched only when the work ahead has completed (see pdl_wait)
     int seg_rows;                     // > 0: the x-marching kernel, segments of this many rows (a multiple of 16);
                                       // 0: one CTA per 32 x 64 tile; -1: the tile kernel with a dynamic queue
     int nsm;                          // SMs of the device (persistent grid of the queue form)
