@@ -388,7 +388,7 @@ int run_forward_loop(ouc_ctx* ctx, int n, bool record, bool save, bool snaps) {
         }
     }
     if (f16) {   // the last slot: its maxima are complete now
-        launch_strip_pack(ctx->d_desc, n, ctx->nt - 1, ctx->ring.R, ctx->strip_slot, ctx->stream);
+        launch_strip_pack(ctx->d_desc, n, ctx->nt - 1, ctx->strip_slot, ctx->stream);
         ctx->timing.kernel_launches += 1;
     }
     ctx->src = s;

@@ -377,21 +377,21 @@ __global__ void k_finalize(const FinalizeArgs f) {
 
 // Conversion of one f16 strip slot from the staging ring once its field
 // maxima are complete (the forward step converts slot t-1 itself; this
-// converts the last slot).  blockIdx.y = shot.
-__global__ void k_strip_pack(const ShotDesc* shots, int slot, int ring, size_t strip_slot) {
+// converts the last slot).  blockIdx.y = shot; a shot's fields follow each
+// other at its own ring's length, shorter than the context's on a sub-grid.
+__global__ void k_strip_pack(const ShotDesc* shots, int slot) {
     const ShotDesc& d = shots[blockIdx.y];
-    const float* src = d.stage + (size_t)(slot & 1) * strip_slot;
-    __half* dst = reinterpret_cast<__half*>(d.strips) + (size_t)slot * strip_slot;
+    const size_t ring = d.ring.R, n = kStripFields * ring;
+    const float* src = d.stage + (size_t)(slot & 1) * d.strip_slot;
+    __half* dst = reinterpret_cast<__half*>(d.strips) + (size_t)slot * d.strip_slot;
     const unsigned* am = d.amax + (size_t)slot * kStripFields;
-    for (size_t e = threadIdx.x + (size_t)blockIdx.x * blockDim.x; e < strip_slot; e += (size_t)blockDim.x * gridDim.x) {
-        const int f = (int)(e / ring);
-        dst[e] = __float2half_rn(scale2(src[e], f16_exp(am[f])));
-    }
+    for (size_t e = threadIdx.x + (size_t)blockIdx.x * blockDim.x; e < n; e += (size_t)blockDim.x * gridDim.x)
+        dst[e] = __float2half_rn(scale2(src[e], f16_exp(am[e / ring])));
 }
 
-void launch_strip_pack(const ShotDesc* shots, int nshots, int slot, int ring, size_t strip_slot, cudaStream_t s) {
-    const int blocks = (int)std::min<size_t>((strip_slot + 255) / 256, 1184);
-    k_strip_pack<<<dim3(blocks, nshots), 256, 0, s>>>(shots, slot, ring, strip_slot);
+void launch_strip_pack(const ShotDesc* shots, int nshots, int slot, size_t strip_slot, cudaStream_t s) {
+    const int blocks = (int)std::min<size_t>((strip_slot + 255) / 256, 1184);   // of the widest possible shot
+    k_strip_pack<<<dim3(blocks, nshots), 256, 0, s>>>(shots, slot);
 }
 
 // ---- source-wavefield snapshots ---------------------------------------------

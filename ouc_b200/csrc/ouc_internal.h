@@ -305,7 +305,7 @@ void launch_finite_check(const float* p, size_t n, int* status, cudaStream_t s);
 // Dense [nf][X][Z] copies of pitched fields, or of the sums f[k] + g[k] where g[k] is given.
 void launch_pack_fields(const float* const* f, int nf, int X, int Z, int pitch, float* out, cudaStream_t s,
                         const float* const* g = nullptr);
-void launch_strip_pack(const ShotDesc* shots, int nshots, int slot, int ring, size_t strip_slot, cudaStream_t s);
+void launch_strip_pack(const ShotDesc* shots, int nshots, int slot, size_t strip_slot, cudaStream_t s);
 void launch_snap_store(const SnapArgs& a, int nshots, cudaStream_t s);
 void launch_image_snap(const SnapArgs& a, int nshots, cudaStream_t s);
 void launch_grad(const GradArgs& a, cudaStream_t s);
