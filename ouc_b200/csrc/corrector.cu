@@ -23,8 +23,8 @@
 // pass) the ReLU mask of the forward activation.
 //
 // Every wait is bounded: an mbarrier that does not complete within ~2 s
-// sets the network's error flag; the CTA then waits once more (also
-// bounded) and releases its tensor memory.
+// sets the network's error flag; the CTA then waits for the multiplications
+// it has committed (also bounded, run_items) and releases its tensor memory.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -38,6 +38,7 @@
 
 #include "../../include/ouc.h"
 #include "../../include/ouc_corrector.h"
+#include "pipeline.h"
 
 namespace ouc {
 namespace cnn {
@@ -209,6 +210,10 @@ struct Items {
         h = (rest - img * row_blocks) * RB;
         z0 = tw * kTile;
     }
+    // items of this CTA: blockIdx.x, then every gridDim.x-th
+    __device__ __forceinline__ int of_cta() const {
+        return count > (int)blockIdx.x ? (count - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    }
 };
 
 // This thread's copies have landed: make them visible to the tensor core's
@@ -278,6 +283,7 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const Items<kCB> items(a.n, a.H, a.W);
+    const int mine = items.of_cta();
 
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
@@ -315,12 +321,12 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
         if (k > 0 && ok) hand_over(&full[(k - 1) & 1]);
     } else if (tid == 128) {   // MMAs
         const uint64_t bd0 = umma_desc(smem_u32(s_w), 5 * COUT * 16, 128);
-        int k = 0;
-        for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
-            const int s = k & 1;
+        const auto ready = [&](int k) {
             const uint32_t ph = (uint32_t)(k >> 1) & 1u;
-            ok = (k < 2 || mbar_wait(&drained[s], ph ^ 1u)) && mbar_wait(&full[s], ph);
-            if (!ok) break;
+            return (k < 2 || mbar_wait(&drained[k & 1], ph ^ 1u)) && mbar_wait(&full[k & 1], ph);
+        };
+        const auto issue = [&](int k) {
+            const int s = k & 1;
             tc_fence_after();
             // descriptors: the start address (in 16-byte units) is the low
             // field, so a tap or chunk is one addition
@@ -344,9 +350,8 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_conv5(const ConvArgs a) {
                 }
             }
             umma_commit(&done[s]);
-        }
-        // the last commits complete before the tensor memory is freed
-        for (int q = k - 2 > 0 ? k - 2 : 0; q < k; ++q) ok = mbar_wait(&done[q & 1], (uint32_t)(q >> 1) & 1u) && ok;
+        };
+        ok = run_items(mine, ready, issue, [&](int s, uint32_t parity) { return mbar_wait(&done[s], parity); });
     } else if (warp < 4) {   // epilogue
         int k = 0;
         for (int it = blockIdx.x; it < items.count; it += gridDim.x, ++k) {
@@ -457,7 +462,7 @@ struct WgradGeo {
     static constexpr int g_bytes = kRB * (COUT / 8) * kTile * 16;  // one stage
     static constexpr int oG = 2 * p_bytes + slack;
     static constexpr int bytes = oG + 2 * g_bytes;
-    static_assert(row_bytes % 128 == 0 && oG % 128 == 0, "tensor-copy destinations are 128-byte aligned");
+    static_assert(row_bytes % 128 == 0 && oG % 128 == 0, "operand rows start on 128-byte boundaries");
     static constexpr int ncols = 5 * NRG * COUT;        // accumulator columns
     static constexpr int tmem_cols = ncols <= 32 ? 32 : ncols <= 64 ? 64 : ncols <= 128 ? 128 : ncols <= 256 ? 256 : 512;
     static_assert(ncols <= 512, "accumulators fit tensor memory");
@@ -487,7 +492,7 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_wgrad_tc(int n, int H, int 
     __shared__ uint32_t tmem_base;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const Items<kRB> items(n, H, W);
-    const int mine = items.count > (int)blockIdx.x ? (items.count - 1 - blockIdx.x) / gridDim.x + 1 : 0;   // items of this CTA
+    const int mine = items.of_cta();
 
     if (tid == 0)
         for (int s = 0; s < 2; ++s) {
@@ -517,10 +522,9 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_wgrad_tc(int n, int H, int 
     } else if (tid == 128) {   // MMAs
         constexpr uint32_t idesc = idesc_bf16_mn(128, COUT);
         uint32_t acc = 0;
-        for (int k = 0; k < mine; ++k) {
+        const auto ready = [&](int k) { return mbar_wait(&full[k & 1], (uint32_t)(k >> 1) & 1u); };
+        const auto issue = [&](int k) {
             const int s = k & 1;
-            ok = mbar_wait(&full[s], (uint32_t)(k >> 1) & 1u);
-            if (!ok) break;
             tc_fence_after();
             int img, h, z0;
             items.at(blockIdx.x + k * gridDim.x, img, h, z0);
@@ -544,8 +548,8 @@ __global__ void __launch_bounds__(kThreadsConv, 1) k_wgrad_tc(int n, int H, int 
                 }
             }
             umma_commit(&done[s]);
-        }
-        for (int q = mine - 2 > 0 ? mine - 2 : 0; q < mine && ok; ++q) ok = mbar_wait(&done[q & 1], (uint32_t)(q >> 1) & 1u);
+        };
+        ok = run_items(mine, ready, issue, [&](int s, uint32_t parity) { return mbar_wait(&done[s], parity); });
     }
     if (!ok) atomicExch(err, 1);
     tc_fence_before();
