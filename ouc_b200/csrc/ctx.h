@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "../../include/ouc.h"
+#include "hostcopy.h"
 #include "ouc_internal.h"
 
 namespace ouc {
@@ -152,11 +153,6 @@ int run_forward_loop(ouc_ctx* ctx, int n, bool record, bool save, bool snaps);
 // stream or `st` (hostio.cu).  As with cudaMemcpyAsync, pageable host arrays
 // may be reused on return when they are the source, and are complete after a
 // synchronisation when they are the destination.
-struct HostCopy {
-    void* host;
-    void* dev;
-    size_t bytes;
-};
 int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st = nullptr);
 inline int to_host(ouc_ctx* ctx, void* dst, const void* src, size_t bytes) {
     return copy_host(ctx, {{dst, const_cast<void*>(src), bytes}}, true);

@@ -13,9 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <atomic>
-#include <cstring>
 #include <new>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -38,12 +36,6 @@ namespace {
 constexpr size_t kTouch = 4 << 20;    // totals from which the pages are touched by a team
 constexpr size_t kRing = 32 << 20;    // totals from which the copies go through the pinned ring
 constexpr int kThreadsMax = 6;
-
-struct Chunk {
-    char* host;
-    char* dev;
-    size_t bytes;
-};
 
 HostRing* ring_of(ouc_ctx* ctx) {
     if (ctx->io) return ctx->io;
@@ -98,7 +90,7 @@ void touch_pages(const std::vector<HostCopy>& copies) {
     size_t total = 0;
     for (const auto& x : copies) total += x.bytes;
     if (total < kTouch) return;
-    std::vector<Chunk> blocks;
+    std::vector<HostCopy> blocks;
     for (const auto& x : copies)
         for (size_t o = 0; o < x.bytes; o += kBlock)
             blocks.push_back({static_cast<char*>(x.host) + o, nullptr, x.bytes - o < kBlock ? x.bytes - o : kBlock});
@@ -106,17 +98,11 @@ void touch_pages(const std::vector<HostCopy>& copies) {
     auto worker = [&]() {
         for (size_t k; (k = next.fetch_add(1)) < blocks.size();)
             for (size_t o = 0; o < blocks[k].bytes; o += kPage) {   // each byte written back as it is
-                volatile char* q = blocks[k].host + o;
+                volatile char* q = static_cast<char*>(blocks[k].host) + o;
                 *q = *q;
             }
     };
-    std::vector<std::thread> team;
-    try {
-        for (int t = 0; t < team_size(); ++t) team.emplace_back(worker);
-    } catch (const std::system_error&) {
-        // fewer threads, or none: the copy takes the remaining faults itself
-    }
-    for (auto& t : team) t.join();
+    run_team(team_size(), worker, [] {});   // without threads the copy takes the faults itself
 }
 
 int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st) {
@@ -134,48 +120,18 @@ int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, c
     if (!ring) return copy_direct(ctx, copies, true, st);
     const cudaError_t ready = cudaStreamSynchronize(st);   // one thread waits for the work ahead, not the whole team
     if (ready != cudaSuccess) return cuda_fail(ctx, ready, "host copy");
-    std::vector<Chunk> chunks;
-    for (const auto& x : copies)
-        for (size_t o = 0; o < x.bytes; o += HostRing::kChunk)
-            chunks.push_back({static_cast<char*>(x.host) + o, static_cast<char*>(x.dev) + o,
-                              x.bytes - o < HostRing::kChunk ? x.bytes - o : HostRing::kChunk});
-    const int n = (int)chunks.size();
-    // chunk k lives in slot k % kSlots.  moved[s] counts the chunks of slot s
-    // that the workers have moved on, queued the chunks whose copies into the
-    // ring have been queued.
-    constexpr int S = HostRing::kSlots;
-    std::atomic<int> moved[S], queued{0}, next{0}, failed{0};
-    for (auto& m : moved) m = 0;
-    auto worker = [&]() {
-        cudaSetDevice(ctx->device);
-        for (int k; (k = next.fetch_add(1)) < n;) {
-            const int s = k % S;
-            while (queued.load(std::memory_order_acquire) <= k && !failed) std::this_thread::yield();
-            if (failed || cudaEventSynchronize(ring->ev[s]) != cudaSuccess) { failed = 1; return; }
-            memcpy(chunks[k].host, ring->mem + (size_t)s * HostRing::kChunk, chunks[k].bytes);
-            moved[s].fetch_add(1, std::memory_order_release);
-        }
-    };
-    std::vector<std::thread> team;
-    try {
-        for (int t = 0; t < team_size() && t < n; ++t) team.emplace_back(worker);
-    } catch (const std::system_error&) {
-        if (team.empty()) return copy_direct(ctx, copies, true, st);   // no threads to be had
-    }
-    cudaError_t err = cudaSuccess;
-    for (int k = 0; k < n && err == cudaSuccess && !failed; ++k) {
-        const int s = k % S;
-        while (moved[s].load(std::memory_order_acquire) < k / S && !failed) std::this_thread::yield();
-        if (failed) break;
-        err = cudaMemcpyAsync(ring->mem + (size_t)s * HostRing::kChunk, chunks[k].dev, chunks[k].bytes,
-                              cudaMemcpyDeviceToHost, st);
-        if (err == cudaSuccess) err = cudaEventRecord(ring->ev[s], st);
-        if (err == cudaSuccess) queued.store(k + 1, std::memory_order_release);
-        else failed = 1;
-    }
-    for (auto& t : team) t.join();
-    if (err != cudaSuccess || failed) return cuda_fail(ctx, err != cudaSuccess ? err : cudaGetLastError(), "host copy");
-    return OUC_OK;
+    const int e = ring_copy(
+        copies, ring->mem, HostRing::kChunk, HostRing::kSlots, team_size(),
+        [&](int s, void* dev, size_t bytes) -> int {
+            const cudaError_t q = cudaMemcpyAsync(ring->mem + (size_t)s * HostRing::kChunk, dev, bytes, cudaMemcpyDeviceToHost, st);
+            return q != cudaSuccess ? q : cudaEventRecord(ring->ev[s], st);
+        },
+        [&](int s) -> int {
+            cudaSetDevice(ctx->device);   // of the calling thread
+            return cudaEventSynchronize(ring->ev[s]);
+        });
+    if (e < 0) return copy_direct(ctx, copies, true, st);   // no threads to be had
+    return e ? cuda_fail(ctx, (cudaError_t)e, "host copy") : OUC_OK;
 }
 
 int records_in(ouc_ctx* ctx, const std::vector<Record>& recs, bool host, cudaStream_t st) {
