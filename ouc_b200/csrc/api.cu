@@ -587,7 +587,7 @@ int finalize(ouc_ctx* ctx, int n) {
     return OUC_OK;
 }
 
-int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host) {
+int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host, bool touched) {
     const size_t n = (size_t)ctx->nt * ctx->X;
     const bool xt = ctx->cfg.gather_layout == OUC_GATHER_XT;
     const float* from = src_tx;
@@ -598,21 +598,20 @@ int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host) {
         from = tgt;
         if (!host) return OUC_OK;
     }
-    if (host) return to_host(ctx, dst, from, n * 4);
+    if (host) return to_host(ctx, dst, from, n * 4, touched);
     CK(cudaMemcpyAsync(dst, from, n * 4, cudaMemcpyDeviceToDevice, ctx->stream));
     return OUC_OK;
 }
 
-int fields_out(ouc_ctx* ctx, const Side& s, float* fields) {
+int fields_out(ouc_ctx* ctx, const Side& s, float* fields, bool touched) {
     const float* f[4] = {s.now[0], s.now[1], s.now[2], s.now[3]};
     const size_t C = (size_t)ctx->X * ctx->Z;
     int rc;
-    touch_pages({{fields, nullptr, 6 * C * 4}});   // while the time loop runs
     launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
-    if ((rc = to_host(ctx, fields + 2 * C, ctx->staging, 4 * C * 4))) return rc;
+    if ((rc = to_host(ctx, fields + 2 * C, ctx->staging, 4 * C * 4, touched))) return rc;
     launch_pack_fields(f, 2, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream, f + 2);   // P + S
     CK(cudaGetLastError());
-    return to_host(ctx, fields, ctx->staging, 2 * C * 4);
+    return to_host(ctx, fields, ctx->staging, 2 * C * 4, touched);
 }
 
 float elapsed(cudaEvent_t a, cudaEvent_t b) {
@@ -1038,9 +1037,13 @@ static int forward_impl(ouc_ctx* ctx, const ouc_shot* shot, const float* wavelet
     launch_finite_check(ctx->gather(0, 0), 2 * (size_t)ctx->nt * ctx->X, ctx->d_status, ctx->stream);
     launch_finite_check(ctx->src.now[0] - (size_t)kGX * ctx->pitch - kZOFF, ctx->fstride, ctx->d_status, ctx->stream);
     CK(cudaEventRecord(ctx->ev[2], ctx->stream));
-    if (gx && (rc = gather_out(ctx, ctx->gather(0, 0), gx, host))) return rc;
-    if (gz && (rc = gather_out(ctx, ctx->gather(0, 1), gz, host))) return rc;
-    if (fields && host && (rc = fields_out(ctx, ctx->src, fields))) return rc;
+    // the results' pages while the time loop runs: the first copy below returns after it
+    const size_t ng = (size_t)ctx->nt * ctx->X * 4;
+    const bool touched = host && touch_pages({{gx, nullptr, ng}, {gz, nullptr, ng},
+                                              {fields, nullptr, (size_t)6 * ctx->X * ctx->Z * 4}});
+    if (gx && (rc = gather_out(ctx, ctx->gather(0, 0), gx, host, touched))) return rc;
+    if (gz && (rc = gather_out(ctx, ctx->gather(0, 1), gz, host, touched))) return rc;
+    if (fields && host && (rc = fields_out(ctx, ctx->src, fields, touched))) return rc;
     CK(cudaEventRecord(ctx->ev[3], ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     if ((rc = check_status(ctx))) return rc;
@@ -1326,7 +1329,8 @@ int ouc_step_fields(ouc_ctx* ctx, int side, float* fields) {
     if (!fields || (side != 0 && side != 1)) return fail(ctx, OUC_EINVAL, "fields is NULL or side is not 0/1");
     if (ctx->step_phase == ouc_ctx::kIdle) return fail(ctx, OUC_ESTATE, "no shot is being stepped");
     cudaSetDevice(ctx->device);
-    const int rc = fields_out(ctx, side == 0 ? ctx->src : ctx->rcv, fields);
+    const bool touched = touch_pages({{fields, nullptr, (size_t)6 * ctx->X * ctx->Z * 4}});
+    const int rc = fields_out(ctx, side == 0 ? ctx->src : ctx->rcv, fields, touched);
     if (rc) return rc;
     CK(cudaStreamSynchronize(ctx->stream));
     return OUC_OK;

@@ -153,13 +153,16 @@ int run_forward_loop(ouc_ctx* ctx, int n, bool record, bool save, bool snaps);
 // stream or `st` (hostio.cu).  As with cudaMemcpyAsync, pageable host arrays
 // may be reused on return when they are the source, and are complete after a
 // synchronisation when they are the destination.
-int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st = nullptr);
-inline int to_host(ouc_ctx* ctx, void* dst, const void* src, size_t bytes) {
-    return copy_host(ctx, {{dst, const_cast<void*>(src), bytes}}, true);
+// touched: the caller has touched the destination's pages (touch_pages).
+int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st = nullptr, bool touched = false);
+inline int to_host(ouc_ctx* ctx, void* dst, const void* src, size_t bytes, bool touched = false) {
+    return copy_host(ctx, {{dst, const_cast<void*>(src), bytes}}, true, nullptr, touched);
 }
 void free_ring(ouc_ctx* ctx);
-// Take the page faults of large host destinations ahead of their copies.
-void touch_pages(const std::vector<HostCopy>& copies);
+// Take the page faults of host destinations ahead of their copies (null ones
+// left out), when together they are large: called once for all results of a
+// call, when the work that makes them has been queued.  Whether it did.
+bool touch_pages(std::vector<HostCopy> arrays);
 // Records of the caller's layout into time-major device gathers of width X,
 // on the context's stream or `st`; host: from host memory.
 struct Record {
@@ -175,8 +178,8 @@ int records_in(ouc_ctx* ctx, const std::vector<Record>& recs, bool host, cudaStr
 int records_fence(ouc_ctx* ctx);
 int records_beside(ouc_ctx* ctx, const std::vector<Record>& recs, bool host);
 // Displacement of a wavefield, (6, X, Z): Ux = P + S, Uz, Px, Pz, Sx, Sz (PS:302-303).
-int fields_out(ouc_ctx* ctx, const Side& s, float* fields);
-int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host);
+int fields_out(ouc_ctx* ctx, const Side& s, float* fields, bool touched);
+int gather_out(ouc_ctx* ctx, const float* src_tx, float* dst, bool host, bool touched = false);
 int ensure_strips(ouc_ctx* ctx);
 int run_backward(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src);
 int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src);

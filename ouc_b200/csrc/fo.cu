@@ -623,7 +623,7 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     const cudaError_t le = cudaGetLastError();   // launch-configuration errors are not reported by the sync
     if (le != cudaSuccess) return cuda_fail(ctx, le, "first-order step launch");
     if (fields) {
-        touch_pages({{fields, nullptr, 16 * C * 4}});   // while the time loop runs
+        const bool touched = touch_pages({{fields, nullptr, 16 * C * 4}});   // while the time loop runs
         // the newest level: written by the last step
         const bool last_even = ((ctx->nt - 1) & 1) == 0;
         const float* v[4];
@@ -635,15 +635,15 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
         const int dst[12] = {2, 3, 4, 5, 8, 9, 10, 11, 12, 13, 14, 15};
         for (int k = 0; k < 12; k += 4) {
             launch_pack_fields(order + k, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream);
-            if ((rc = to_host(ctx, fields + (size_t)dst[k] * C, ctx->staging, 4 * C * 4))) return rc;   // 4 fields in a row
+            if ((rc = to_host(ctx, fields + (size_t)dst[k] * C, ctx->staging, 4 * C * 4, touched))) return rc;   // 4 fields in a row
         }
         // totals as the kernels form them: U = P + S, theta = theta_x +
         // theta_z + s, omega = omega_x + omega_z (the source term below)
         const float* f[4] = {v[0], v[1], st[0], st[2]};
         const float* g[4] = {v[2], v[3], st[1], st[3]};
         launch_pack_fields(f, 4, ctx->X, ctx->Z, ctx->pitch, ctx->staging, ctx->stream, g);
-        if ((rc = to_host(ctx, fields, ctx->staging, 2 * C * 4))) return rc;
-        if ((rc = to_host(ctx, fields + 6 * C, ctx->staging + 2 * C, 2 * C * 4))) return rc;
+        if ((rc = to_host(ctx, fields, ctx->staging, 2 * C * 4, touched))) return rc;
+        if ((rc = to_host(ctx, fields + 6 * C, ctx->staging + 2 * C, 2 * C * 4, touched))) return rc;
     }
     const cudaError_t e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "first-order time loop");

@@ -12,6 +12,7 @@
 // Host memory that is pinned already goes straight to cudaMemcpyAsync.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <atomic>
 #include <new>
 #include <thread>
@@ -85,13 +86,17 @@ void free_ring(ouc_ctx* ctx) {
     ctx->io = nullptr;
 }
 
-void touch_pages(const std::vector<HostCopy>& copies) {
+// Pinned arrays have their pages; only the others are touched.
+bool touch_pages(std::vector<HostCopy> arrays) {
+    arrays.erase(std::remove_if(arrays.begin(), arrays.end(),
+                                [](const HostCopy& x) { return !x.host || x.bytes == 0 || pinned(x.host); }),
+                 arrays.end());
     constexpr size_t kPage = 4096, kBlock = 256 * kPage;
     size_t total = 0;
-    for (const auto& x : copies) total += x.bytes;
-    if (total < kTouch) return;
+    for (const auto& x : arrays) total += x.bytes;
+    if (total < kTouch) return false;
     std::vector<HostCopy> blocks;
-    for (const auto& x : copies)
+    for (const auto& x : arrays)
         for (size_t o = 0; o < x.bytes; o += kBlock)
             blocks.push_back({static_cast<char*>(x.host) + o, nullptr, x.bytes - o < kBlock ? x.bytes - o : kBlock});
     std::atomic<size_t> next{0};
@@ -103,9 +108,10 @@ void touch_pages(const std::vector<HostCopy>& copies) {
             }
     };
     run_team(team_size(), worker, [] {});   // without threads the copy takes the faults itself
+    return true;
 }
 
-int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st) {
+int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, cudaStream_t st, bool touched) {
     if (!st) st = ctx->stream;
     if (!to_host) return copy_direct(ctx, copies, false, st);
     size_t total = 0;
@@ -115,7 +121,7 @@ int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, c
         direct = direct || pinned(x.host);
     }
     if (direct || total < kTouch) return copy_direct(ctx, copies, true, st);
-    touch_pages(copies);
+    if (!touched) touch_pages(copies);
     HostRing* ring = total >= kRing ? ring_of(ctx) : nullptr;
     if (!ring) return copy_direct(ctx, copies, true, st);
     const cudaError_t ready = cudaStreamSynchronize(st);   // one thread waits for the work ahead, not the whole team
