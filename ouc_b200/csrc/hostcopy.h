@@ -1,9 +1,11 @@
 // Host side of large copies from the device (hostio.cu), apart from the CUDA
 // calls so that it also runs without a GPU.
 #pragma once
+#include <algorithm>
 #include <atomic>
 #include <cstddef>
 #include <cstring>
+#include <functional>
 #include <system_error>
 #include <thread>
 #include <vector>
@@ -16,6 +18,15 @@ struct HostCopy {
     void* dev;
     size_t bytes;
 };
+
+// Whether two of the arrays share bytes: their copies must then be made in order.
+inline bool overlapping(std::vector<HostCopy> c) {
+    c.erase(std::remove_if(c.begin(), c.end(), [](const HostCopy& x) { return x.bytes == 0; }), c.end());
+    std::sort(c.begin(), c.end(), [](const HostCopy& a, const HostCopy& b) { return std::less<void*>()(a.host, b.host); });
+    for (size_t k = 1; k < c.size(); ++k)
+        if (std::less<char*>()(static_cast<char*>(c[k].host), static_cast<char*>(c[k - 1].host) + c[k - 1].bytes)) return true;
+    return false;
+}
 
 // Run `worker` on up to n new threads and `caller` on this one, then join
 // them.  Where the system gives fewer threads, those that started do the work;

@@ -122,7 +122,7 @@ int copy_host(ouc_ctx* ctx, const std::vector<HostCopy>& copies, bool to_host, c
     }
     if (direct || total < kTouch) return copy_direct(ctx, copies, true, st);
     if (!touched) touch_pages(copies);
-    HostRing* ring = total >= kRing ? ring_of(ctx) : nullptr;
+    HostRing* ring = total >= kRing && !overlapping(copies) ? ring_of(ctx) : nullptr;
     if (!ring) return copy_direct(ctx, copies, true, st);
     const cudaError_t ready = cudaStreamSynchronize(st);   // one thread waits for the work ahead, not the whole team
     if (ready != cudaSuccess) return cuda_fail(ctx, ready, "host copy");
