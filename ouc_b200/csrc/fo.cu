@@ -35,6 +35,7 @@ struct FoArgs {
     alignas(64) CUtensorMap map;     // U box of the launch's tile over the state block
     int vfield[4];                   // fields of vold[] in the block
     int* err;                        // device status word (bit 0: a copy wait ran out)
+    unsigned copy_tx_extra;          // test hook, as StepArgs::copy_tx_extra
     int X, Z, pitch, tiles_z, t, nt;
     int sx, sz, rz;                  // padded source cell and receiver row
     float a[6];
@@ -185,7 +186,7 @@ __global__ void __launch_bounds__(kThreads, 2) k_fo(const __grid_constant__ FoAr
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         prefetch_map(&p.map);
         pdl_wait();
-        issue_box<G>(&p.map, p.vfield, 0u, sm, x0, z0, 0, &bar);
+        issue_box<G>(&p.map, p.vfield, p.copy_tx_extra, sm, x0, z0, 0, &bar);
     }
     float a[N];
 #pragma unroll
@@ -384,7 +385,7 @@ __global__ void __launch_bounds__(SmallGeo<N, TXr>::NT, CTAS) k_fo_small(const _
     }
     __syncthreads();   // the mbarrier is initialised
     pdl_wait();
-    if (tid == 0) issue_box<G>(&p.map, p.vfield, 0u, sm, x0, z0, 0, &bar);
+    if (tid == 0) issue_box<G>(&p.map, p.vfield, p.copy_tx_extra, sm, x0, z0, 0, &bar);
     if (has_s) {
         // theta_x omega_x Qxx Qzx | theta_z omega_z Qxz Qzz
 #pragma unroll
@@ -595,6 +596,7 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     a.wavelet = backward ? nullptr : ctx->d_wavelet;
     a.err = ctx->d_status;
     const StepArgs b = base_args(ctx);
+    a.copy_tx_extra = b.copy_tx_extra;
     const Tier tier = pick_tier(ctx->N, nullptr, &b, kFwd, 1);
     a.map = tier == kLarge ? b.box_map : tier == kMid ? b.mid_map : b.small_map[tier == kSmall24 ? 1 : 0];
     auto field_of = [&](const float* f) { return (int)((f - ctx->field(ctx->state, 0)) / (ptrdiff_t)ctx->fstride); };
