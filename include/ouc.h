@@ -329,6 +329,14 @@ int ouc_get_step_kernel(const ouc_ctx* ctx, int* seg_rows);
  * captured time loops. */
 int ouc_debug_copy_stall(ouc_ctx* ctx, int on);
 
+/* Test hook: the tile shape of the tile kernels' launches (second and first
+ * order), which otherwise follows from the number of tiles.  0 (the default):
+ * by that rule; 1: 32 x 64 cells; 2: 16 x 64; 3: 24 x 32; 4 and 5: 16 x 32,
+ * two CTAs per SM and one.  The results do not depend on it.  OUC_EINVAL for
+ * any other value and where the context's fields do not hold 24-row tiles.
+ * Drops the captured time loops. */
+int ouc_debug_tile_shape(ouc_ctx* ctx, int shape);
+
 /* Device time of one launch of each step kernel at batch n (ms[0] forward,
  * ms[1] receiver, ms[2] reconstruction + imaging), averaged over `reps`
  * launches after one warm-up, on the state the last RTM batch of n shots

@@ -386,6 +386,11 @@ class Context:
         copy waits run out, so that the next call reports OUC_ETIMEOUT."""
         check(lib().ouc_debug_copy_stall(self._h, int(bool(on))), self._h)
 
+    def debug_tile_shape(self, shape):
+        """Test hook (ouc_debug_tile_shape): the tile kernels' tile shape, 1 .. 5;
+        0: by the number of tiles."""
+        check(lib().ouc_debug_tile_shape(self._h, int(shape)), self._h)
+
     def step_kernel(self):
         v = C.c_int()
         check(lib().ouc_get_step_kernel(self._h, C.byref(v)), self._h)

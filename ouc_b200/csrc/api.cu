@@ -176,6 +176,7 @@ StepArgs base_args(const ouc_ctx* c) {
     a.fstride = c->fstride;
     a.nfields = kFieldsPerShot;
     a.copy_tx_extra = c->copy_stall ? 16u : 0u;
+    a.tier = c->tile_shape;
     return a;
 }
 
@@ -488,10 +489,10 @@ int run_backward_loop(ouc_ctx* ctx, int n, bool exact_strips, bool theta_src) {
     if (ctx->cfg.gradient) CK(cudaMemsetAsync(ctx->grad, 0, (size_t)n * 3 * ctx->fstride * sizeof(float), ctx->stream));
     StepArgs ar = rcv_args(ctx);
     StepArgs as = rec_args(ctx);
-    Tier tier = kAuto;
-    if (ctx->seg_rows == 0) tier = pick_tier(ctx->N, &as, &ar, kRcv, n);
+    Tier tier = (Tier)ctx->tile_shape;
+    if (tier == kAuto && ctx->seg_rows == 0) tier = pick_tier(ctx->N, &as, &ar, kRcv, n);
     ar.tier = as.tier = tier;
-    if (tier >= kSmall24) {
+    if (tier >= kSmall24 && ctx->seg_rows == 0) {
         // Small launches: one per back-step holds the reconstruction +
         // imaging of step t+1 and the receiver step t, which are independent
         // (k_small_back).  The gradient of step t+1 reads both sides first.
@@ -988,6 +989,19 @@ int ouc_debug_copy_stall(ouc_ctx* ctx, int on) {
     for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.exec);
     ctx->graphs.clear();
     ctx->copy_stall = on != 0;
+    return OUC_OK;
+}
+
+int ouc_debug_tile_shape(ouc_ctx* ctx, int shape) {
+    if (!ctx || shape < kAuto || shape > kSmall16) return OUC_EINVAL;
+    const StepArgs full = rcv_args(ctx), rec = rec_args(ctx);
+    if (shape == kSmall24 && !(fits24(kRcv, full, ctx->N) && fits24(kRec, rec, ctx->N)))
+        return fail(ctx, OUC_EINVAL, "the fields do not hold 24-row tiles");
+    cudaSetDevice(ctx->device);
+    if (ctx->stream) cudaStreamSynchronize(ctx->stream);
+    for (auto& g : ctx->graphs) cudaGraphExecDestroy(g.exec);
+    ctx->graphs.clear();
+    ctx->tile_shape = shape;
     return OUC_OK;
 }
 

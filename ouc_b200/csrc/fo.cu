@@ -597,7 +597,7 @@ int fo_run(ouc_ctx* ctx, const ouc_shot* shot, bool backward, float theta_src, f
     a.err = ctx->d_status;
     const StepArgs b = base_args(ctx);
     a.copy_tx_extra = b.copy_tx_extra;
-    const Tier tier = pick_tier(ctx->N, nullptr, &b, kFwd, 1);
+    const Tier tier = b.tier != kAuto ? (Tier)b.tier : pick_tier(ctx->N, nullptr, &b, kFwd, 1);
     a.map = tier == kLarge ? b.box_map : tier == kMid ? b.mid_map : b.small_map[tier == kSmall24 ? 1 : 0];
     auto field_of = [&](const float* f) { return (int)((f - ctx->field(ctx->state, 0)) / (ptrdiff_t)ctx->fstride); };
     float* gx = ctx->gather(0, 0);

@@ -71,7 +71,7 @@ static Grid grid_of(Mode mode, const StepArgs& a, int TX, int TZ) {
     return g;
 }
 // 24-row tiles may end beyond the rows the field allocation keeps for 32-row ones.
-static bool fits24(Mode mode, const StepArgs& a, int N) {
+bool fits24(Mode mode, const StepArgs& a, int N) {
     const int rows = mode == kRec ? a.X - 2 * a.L : a.X, x0 = mode == kRec ? a.tile_x0 : 0;
     return x0 + (rows + 23) / 24 * 24 + N <= (int)(a.fstride / a.pitch) - kGX;
 }

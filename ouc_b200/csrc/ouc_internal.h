@@ -290,6 +290,8 @@ cudaError_t encode_box_map(StepArgs& a, const float* state0, int pitch, int rows
 int launch_step(int N, Mode mode, const StepArgs& a, int tiles_x, int nshots, cudaStream_t s);
 // Tile shape of a launch of `mode`, run beside a reconstruction launch when rec is given.
 Tier pick_tier(int N, const StepArgs* rec, const StepArgs* other, Mode mode, int nshots);
+// Whether 24-row tiles stay inside the fields of a launch of `mode`.
+bool fits24(Mode mode, const StepArgs& a, int N);
 int launch_back(int N, const StepArgs& rec, const StepArgs& rcv, int nshots, cudaStream_t s);
 // Segments of the x-marching kernel for a launch (rows of the widest shot).
 int march_segments(Mode mode, const StepArgs& a);
