@@ -35,7 +35,6 @@ struct FoArgs {
     alignas(64) CUtensorMap map;     // U box of the launch's tile over the state block
     int vfield[4];                   // fields of vold[] in the block
     int* err;                        // device status word (bit 0: a copy wait ran out)
-    unsigned copy_tx_extra;          // test hook, as StepArgs::copy_tx_extra
     int X, Z, pitch, tiles_z, t, nt;
     int sx, sz, rz;                  // padded source cell and receiver row
     float a[6];
@@ -54,6 +53,7 @@ struct FoArgs {
     const float* inj_x;              // records injected into U at the receiver
     const float* inj_z;              // row on [L, X-L) (row t), or null
     int L;
+    unsigned copy_tx_extra;          // test hook, as StepArgs::copy_tx_extra
 };
 
 // split-field stress update, the reference's expression (PS:547-556)
