@@ -926,7 +926,7 @@ int ouc_cnn_backward_dev(ouc_cnn* net, const float* d_gout, void* stream) {
             cudaSuccess)
             return OUC_ECUDA;
         k_bgrad<32><<<kBgradBlocks, 256, 0, s>>>(P, gl, net->bpart);
-    k_grad_sum<<<kTaps * kMaxPairs / 32 + 4, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l), kBgradBlocks, net->bpart,
+        k_grad_sum<<<kTaps * kMaxPairs / 32 + 4, 256, 0, s>>>(nb, kL[l].cin, kL[l].cout, net->part, gp + p_offset(l), kBgradBlocks, net->bpart,
                                    gp + p_offset(l) + w_count(l));
         a.x = gl; a.w = net->wd[l]; a.mask = net->y[l - 1]; a.y = net->g[(3 - l) & 1];
         if (launch_conv<32, 32, kDgrad>(a, net->sms, s) != cudaSuccess) return OUC_ECUDA;

@@ -161,7 +161,7 @@ __device__ __forceinline__ float4 neg4(float4 v) { return make_float4(-v.x, -v.y
 
 // Bound: latency and issue, as the second-order step.  1060 x 560, per step:
 // 32 x 64 tiles with plain loads 52 us; 16 x 64 tiles, tensor copies and
-// operands ahead of the derivatives 32 us (40 us before inside a time loop).
+// operands ahead of the derivatives 33 us (40 us before inside a time loop).
 template <int N, class G>
 __global__ void __launch_bounds__(kThreads, 2) k_fo(const __grid_constant__ FoArgs p) {
     constexpr int TX = G::TX, TZ = G::TZ, SHX = G::SHX, HS = G::HS, HU = G::HU, UC = G::UC, SC = G::SC;
